@@ -33,6 +33,29 @@ __device__ __forceinline__ float hs_scan_n(float x, int lane, int steps)
     return x;
 }
 
+// one Hillis-Steele step: lanes below `off` keep x
+__device__ __forceinline__ float hs_up(float x, int off)
+{
+    float r;
+    asm volatile("{\n .reg .pred p;\n .reg .f32 y;\n"
+                 " shfl.sync.up.b32 y|p, %1, %2, 0, 0xffffffff;\n"
+                 " mov.f32 %0, %1;\n"
+                 " @p add.rn.f32 %0, %1, y;\n}"
+                 : "=&f"(r) : "f"(x), "r"(off));
+    return r;
+}
+
+// the value of the lane before, 0 in lane 0
+__device__ __forceinline__ float up1_or_0(float x)
+{
+    float r;
+    asm volatile("{\n .reg .pred p;\n .reg .f32 y;\n"
+                 " shfl.sync.up.b32 y|p, %1, 1, 0, 0xffffffff;\n"
+                 " selp.f32 %0, y, 0f00000000, p;\n}"
+                 : "=f"(r) : "f"(x));
+    return r;
+}
+
 __host__ __device__ __forceinline__ uint32_t round4(uint32_t x) { return (x + 3u) & ~3u; }
 
 __device__ __forceinline__ double warp_sum(double x)

@@ -935,6 +935,8 @@ k_sweep_doc(SweepArgs a)
     }
 }
 
+#include "sweep_reg.cuh"
+
 // ---------------------------------------------------------------------------
 // log-likelihood in FP64 (getLLDocs / getLLRest, LDAModel.hpp:616-668)
 // ---------------------------------------------------------------------------
@@ -1635,21 +1637,15 @@ void launch_sweep_t(tmt_handle* h, const SweepArgs& a, const SweepShape& sh)
 // two of the tuner's sweeps spent on it; at K = 1000, the word's column
 // read from L1 every token, 6 blocks/SM, and a per-warp shared-memory copy
 // of it -- fewer instructions, slower sweeps.)
+// K <= kRegMaxK (k_sweep_reg) and K > 4096 have one variant.
 int sweep_variants_for(uint32_t K)
 {
-    return (round4(K) + 127) / 128 > 32 ? 1 : 2;
+    return K <= kRegMaxK || (round4(K) + 127) / 128 > 32 ? 1 : 2;
 }
 
 template <int CH, bool WT, bool PLAIN>
 void launch_sweep_cp(tmt_handle* h, const SweepArgs& a, const SweepShape& sh, int variant)
 {
-    // split documents: integer counts, up to 4 blocks of four topics per lane
-    constexpr bool kSplit = !WT && CH >= 1 && CH <= 4;
-    if (kSplit && a.n_long > 0) {
-        if (variant >= 1) launch_sweep_t<CH, 4, WT, kSplit, PLAIN>(h, a, sh);
-        else launch_sweep_t<CH, 3, WT, kSplit, PLAIN>(h, a, sh);
-        return;
-    }
     if (variant >= 1) {
         if constexpr (!WT) {
             if (sh.row16) return launch_sweep_t<CH, 4, WT, false, PLAIN, true>(h, a, sh);
@@ -1672,17 +1668,62 @@ void launch_sweep_ch(tmt_handle* h, const SweepArgs& a, const SweepShape& sh, in
 template <bool WT>
 void launch_sweep_w(tmt_handle* h, const SweepArgs& b, const SweepShape& sh, uint32_t ch, int variant, bool plain)
 {
-    if (ch <= 1) launch_sweep_ch<1, WT>(h, b, sh, variant, plain);
-    else if (ch <= 2) launch_sweep_ch<2, WT>(h, b, sh, variant, plain);
-    else if (ch <= 4) launch_sweep_ch<4, WT>(h, b, sh, variant, plain);
+    if constexpr (!WT) {
+        // K <= kSplitMaxK with documents of kRegMaxLen tokens or more
+        if (b.n_long) return launch_sweep_t<0, 3, false, true>(h, b, sh);
+    }
+    if (ch <= 4) launch_sweep_t<0, 3, WT>(h, b, sh);     // as above, not split
     else if (ch <= 8) launch_sweep_ch<8, WT>(h, b, sh, variant, plain);
     else if (ch <= 16) launch_sweep_ch<16, WT>(h, b, sh, variant, plain);
     else if (ch <= 32) launch_sweep_ch<32, WT>(h, b, sh, variant, plain);
     else launch_sweep_t<0, 3, WT>(h, b, sh);
 }
 
+// --- k_sweep_reg: K <= kRegMaxK ---
+template <int CH, int STEPS, bool WT, bool SPLIT, bool OPT>
+void launch_reg_t(tmt_handle* h, const SweepArgs& a)
+{
+    auto kern = k_sweep_reg<CH, STEPS, WT, SPLIT, OPT>;
+    const uint32_t warps = SPLIT ? kSweepWarps : kRegWarps;
+    const uint32_t smem = WT ? 0 : 4 * round4(a.K) * (SPLIT ? 4 : 1);      // at most 8 KB
+    int per_sm = 0;
+    for (const auto& e : h->occ)
+        if (e.kern == (const void*)kern && e.smem == smem) per_sm = e.per_sm;
+    if (per_sm == 0) {
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem));
+        if (per_sm < 1) throw CudaError("sweep kernel does not fit on an SM");
+        h->occ.push_back({ (const void*)kern, smem, per_sm });
+    }
+    const uint64_t n_long = SPLIT ? a.n_long : 0;
+    const uint64_t docs = a.pos_end - a.pos_begin - n_long;
+    const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)per_sm * h->num_sms,
+                                                                          n_long + (docs + warps - 1) / warps));
+    kern<<<grid, warps * 32, smem, h->stream>>>(a);
+    launch_check(h);
+}
+
+template <int CH, int STEPS>
+void launch_reg_ch(tmt_handle* h, const SweepArgs& a)
+{
+    const bool opt = a.arow || a.mask;
+    if (a.wt) launch_reg_t<CH, STEPS, true, false, true>(h, a);
+    else if (a.n_long) opt ? launch_reg_t<CH, STEPS, false, true, true>(h, a) : launch_reg_t<CH, STEPS, false, true, false>(h, a);
+    else opt ? launch_reg_t<CH, STEPS, false, false, true>(h, a) : launch_reg_t<CH, STEPS, false, false, false>(h, a);
+}
+
+void launch_reg(tmt_handle* h, const SweepArgs& a)
+{
+    if (a.K <= 32) launch_reg_ch<1, 3>(h, a);
+    else if (a.K <= 64) launch_reg_ch<1, 4>(h, a);
+    else if (a.K <= 128) launch_reg_ch<1, 5>(h, a);
+    else if (a.K <= 256) launch_reg_ch<2, 5>(h, a);
+    else if (a.K <= 384) launch_reg_ch<3, 5>(h, a);
+    else launch_reg_ch<4, 5>(h, a);
+}
+
 void launch_sweep(tmt_handle* h, const SweepArgs& a, int variant)
 {
+    if (a.K <= kRegMaxK && a.max_len < kRegMaxLen) return launch_reg(h, a);
     const uint32_t KP = round4(a.K);
     const uint32_t ch = (KP + 127) / 128;
     const bool wt = a.wt != nullptr;
