@@ -1316,6 +1316,7 @@ struct tmt_handle {
     double* d_llv = nullptr;         // tmt_ll output (2)
     double* d_partials = nullptr;
     uint32_t n_partials = 0;
+    bool nk_ok = true;               // no negative n_k (set_counts may bring some)
     double* d_ll = nullptr;          // ll history for one train() call (2 per point)
     uint32_t ll_cap = 0;
     float* d_dg_points = nullptr;
@@ -1330,6 +1331,7 @@ struct tmt_handle {
         double* ll = nullptr;
         float* acum = nullptr;
         uint32_t* counter = nullptr;
+        uint32_t* work = nullptr;        // documents, longest first
         float* wt = nullptr;
         uint64_t cap_wt = 0;
     } inf;
@@ -1369,6 +1371,7 @@ struct tmt_handle {
         drop_graphs();
         for (void* p : allocs) cudaFree(p);
         allocs.clear();
+        inf = InferBufs{};          // freed with the rest
         bytes = 0;
     }
 
@@ -2197,6 +2200,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
         }
         h->release();
         h->uploaded = false;
+        h->nk_ok = true;
         h->D = D;
         h->N_all = n_all;
         h->global_step = 0;
@@ -2693,6 +2697,7 @@ tmt_status tmt_set_counts(tmt_handle* h, const int32_t* n_kw, const int32_t* n_k
         const uint64_t kv = (uint64_t)h->cfg.K * h->cfg.V;
         h2d(h, h->d_nkw[h->cur], n_kw, kv * sizeof(int32_t));
         CK(cudaMemcpyAsync(h->d_nk[h->cur], n_k, h->cfg.K * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
+        h->nk_ok = *std::min_element(n_k, n_k + h->cfg.K) >= 0;
         CK(cudaStreamSynchronize(h->stream));
     });
 }
@@ -3036,6 +3041,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
             B.doc_off = h->dalloc<uint64_t>(D + 1);
             B.keys = h->dalloc<uint64_t>(D);
             B.ll = h->dalloc<double>(D);
+            B.work = h->dalloc<uint32_t>(D);
             B.cap_docs = D;
         }
         if (D * K > B.cap_theta) {
@@ -3066,6 +3072,14 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         CK(cudaMemcpyAsync(B.doc_off, doc_off, (D + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
         h2d(h, B.words, sorted.data(), n_all * sizeof(uint32_t));
         if (weights) h2d(h, B.wt, wsorted.data(), n_all * sizeof(float));
+        // longest documents first: a document is one warp's chain, and a long one
+        // taken up last would run on alone
+        std::vector<uint32_t> work(D);
+        std::iota(work.begin(), work.end(), 0u);
+        std::stable_sort(work.begin(), work.end(), [&](uint32_t x, uint32_t y) {
+            return doc_off[x + 1] - doc_off[x] > doc_off[y + 1] - doc_off[y];
+        });
+        CK(cudaMemcpyAsync(B.work, work.data(), D * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         if (doc_keys) CK(cudaMemcpyAsync(B.keys, doc_keys, D * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(B.acum, acum.data(), K * sizeof(float), cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(B.counter, 0, sizeof(uint32_t), st));
@@ -3096,7 +3110,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         a.ndk = nullptr;
         a.theta = B.theta;
         a.ll = B.ll;
-        a.work = nullptr;
+        a.work = B.work;
         a.n_work = (uint32_t)D;
         a.counter = B.counter;
         a.wt = weights ? B.wt : nullptr;
@@ -3105,6 +3119,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         a.esum = h->d_esum;
         a.pcum = h->d_prior_cum;
         a.ecum = h->d_cum_eta;
+        a.nk_ok = h->nk_ok;
         launch_infer(a, h->num_sms, h->stream);
         ++h->launches;
         if (theta) d2h(h, theta, B.theta, D * (uint64_t)K * sizeof(float));

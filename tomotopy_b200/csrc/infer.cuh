@@ -65,7 +65,73 @@ struct InferArgs {
     const float* esum;
     const float* pcum;
     const float* ecum;
+    // the caller's n_k holds no negative value (only counts set from outside can)
+    bool nk_ok;
 };
+
+// A finished document's theta and FP64 ll over the cells it touched.  dlen: its
+// length (weight sum); own: K zeroed ints, zeroed again on return; count(k): its n_dk.
+template <bool WT, class F>
+__device__ __forceinline__ void finish_doc(const InferArgs& a, uint32_t sl, uint64_t b, uint32_t L, float dlen, int lane,
+                                           int* own, F count)
+{
+    using CT = typename std::conditional<WT, float, int>::type;
+    const CT* nkw = reinterpret_cast<const CT*>(a.nkw);
+    const CT* nkv = reinterpret_cast<const CT*>(a.nk);
+    const int K = (int)a.K;
+    double acc = 0;
+    const float denom = __fadd_rn(dlen, a.asum_f);
+    for (int k = lane; k < K; k += 32) {
+        const CT n = count(k);
+        if (a.theta) a.theta[(uint64_t)sl * K + k] = __fdiv_rn(__fadd_rn((float)n, __ldg(a.alpha + k)), denom);
+        if (n != CT(0)) {
+            const double gk = (double)__ldg(nkv + k);
+            const double es = a.esum ? (double)__ldg(a.esum + k) : a.veta_d;
+            acc += lgamma(gk + es) - lgamma(gk + (double)n + es);
+            const double al = (double)__ldg(a.alpha + k);
+            acc += lgamma((double)n + al) - lgamma(al);
+        }
+    }
+    uint32_t rb = 0;
+    while (rb < L) {            // word cells: per run, each distinct topic once
+        const uint32_t v = a.words[b + rb];
+        uint32_t re = rb + 1;
+        for (;;) {
+            const uint32_t j = re + lane;
+            const bool diff = j >= L || a.words[b + j] != v;
+            const unsigned mm = __ballot_sync(FULL, diff);
+            if (mm) { re += __ffs(mm) - 1; break; }
+            re += 32;
+        }
+        if (v < a.V) {
+            for (uint32_t j = rb + lane; j < re; j += 32) atomicAdd(&own[a.z[b + j]], 1);
+            __syncwarp();
+            const float wr = WT ? a.wt[b + rb] : 1.f;    // the run's weight
+            const float* pe = nullptr;
+            if (a.pidx) {
+                const int p = a.pidx[v];
+                if (p >= 0) pe = a.pval + (uint64_t)p * K;
+            }
+            for (uint32_t j = rb + lane; j < re; j += 32) {
+                const int k = a.z[b + j];
+                const int c = atomicExch(&own[k], 0);
+                if (c) {
+                    const CT gk = __ldg(nkw + (uint64_t)v * K + k);
+                    const double ek = pe ? (double)pe[k] : (double)a.eta;
+                    double after;
+                    if constexpr (WT) after = lgamma(((double)gk + (double)__fmul_rn((float)c, wr)) + ek);
+                    else after = lgamma((double)(gk + c) + ek);
+                    acc += after - (gk != CT(0) ? lgamma((double)gk + ek) : (pe ? lgamma(ek) : a.lg_eta));
+                }
+            }
+            __syncwarp();
+        }
+        rb = re;
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && a.ll) a.ll[sl] = acc - (lgamma((double)dlen + a.asum_d) - a.lg_asum);
+    __syncwarp();
+}
 
 // WT: weighted counts.  The document's counts n_dk are float sums of weights
 // (a removal clamps at 0, updateCnt<true>); B_k = (n_kw[k,v] + own[k] * w) + eta
@@ -363,61 +429,11 @@ k_infer_slots(InferArgs a)
             continue;
         }
         // finished: theta, FP64 ll over the touched cells
-        double acc = 0;
-        const float dlen = WT ? wsum : (float)nvalid;
-        const float denom = __fadd_rn(dlen, a.asum_f);
-        for (int k = lane; k < K; k += 32) {
-            const CT n = rowi[k];
-            if (a.theta) a.theta[(uint64_t)sl * K + k] = __fdiv_rn(__fadd_rn((float)n, __ldg(a.alpha + k)), denom);
-            if (n != CT(0)) {
-                const double gk = (double)__ldg(nkv + k);
-                const double es = a.esum ? (double)__ldg(a.esum + k) : a.veta_d;
-                acc += lgamma(gk + es) - lgamma(gk + (double)n + es);
-                const double al = (double)__ldg(a.alpha + k);
-                acc += lgamma((double)n + al) - lgamma(al);
-            }
-        }
-        uint32_t rb = 0;
-        while (rb < L) {            // word cells: per run, each distinct topic once
-            const uint32_t v = a.words[b + rb];
-            uint32_t re = rb + 1;
-            for (;;) {
-                const uint32_t j = re + lane;
-                const bool diff = j >= L || a.words[b + j] != v;
-                const unsigned mm = __ballot_sync(FULL, diff);
-                if (mm) { re += __ffs(mm) - 1; break; }
-                re += 32;
-            }
-            if (v < a.V) {
-                for (uint32_t j = rb + lane; j < re; j += 32) atomicAdd(&own[a.z[b + j]], 1);
-                __syncwarp();
-                const float wr = WT ? a.wt[b + rb] : 1.f;    // the run's weight
-                const float* pe = nullptr;
-                if (a.pidx) {
-                    const int p = a.pidx[v];
-                    if (p >= 0) pe = a.pval + (uint64_t)p * K;
-                }
-                for (uint32_t j = rb + lane; j < re; j += 32) {
-                    const int k = a.z[b + j];
-                    const int c = atomicExch(&own[k], 0);
-                    if (c) {
-                        const CT gk = __ldg(nkw + (uint64_t)v * K + k);
-                        const double ek = pe ? (double)pe[k] : (double)a.eta;
-                        double after;
-                        if constexpr (WT) after = lgamma(((double)gk + (double)__fmul_rn((float)c, wr)) + ek);
-                        else after = lgamma((double)(gk + c) + ek);
-                        acc += after - (gk != CT(0) ? lgamma((double)gk + ek) : (pe ? lgamma(ek) : a.lg_eta));
-                    }
-                }
-                __syncwarp();
-            }
-            rb = re;
-        }
-        acc = warp_sum(acc);
-        if (lane == 0 && a.ll) a.ll[sl] = acc - (lgamma((double)dlen + a.asum_d) - a.lg_asum);
-        __syncwarp();
+        finish_doc<WT>(a, sl, b, L, WT ? wsum : (float)nvalid, lane, own, [&](int k) { return rowi[k]; });
     }
 }
+
+#include "infer_reg.cuh"
 
 // warps per block so that 16 * KP bytes of state per warp fit in 200 KB; 0: too large
 inline uint32_t infer_warps(uint32_t K)
@@ -444,19 +460,55 @@ inline void launch_infer_t(const InferArgs& a, uint32_t warps, int num_sms, cuda
 template <bool WT>
 inline void launch_infer_w(const InferArgs& a, uint32_t warps, uint32_t ch, int num_sms, cudaStream_t st)
 {
-    if (ch <= 1) launch_infer_t<1, WT>(a, warps, num_sms, st);
-    else if (ch <= 2) launch_infer_t<2, WT>(a, warps, num_sms, st);
-    else if (ch <= 4) launch_infer_t<4, WT>(a, warps, num_sms, st);
-    else if (ch <= 8) launch_infer_t<8, WT>(a, warps, num_sms, st);
-    else if (ch <= 16) launch_infer_t<16, WT>(a, warps, num_sms, st);
+    if (ch <= 16) launch_infer_t<16, WT>(a, warps, num_sms, st);
     else if (ch <= 32) launch_infer_t<32, WT>(a, warps, num_sms, st);
     else launch_infer_t<0, WT>(a, warps, num_sms, st);
+}
+
+template <int CH, int STEPS, bool WT, bool GEN>
+inline void launch_infer_reg_t(const InferArgs& a, int num_sms, cudaStream_t st)
+{
+    auto kern = k_infer_reg<CH, STEPS, WT, GEN>;
+    const uint32_t smem = (kInferRegWarps + 1) * 16 * 128 * CH;
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kInferRegWarps * 32, smem));
+    if (per_sm < 1) throw CudaError("infer kernel does not fit on an SM");
+    const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)per_sm * num_sms,
+                                                                          (a.n_work + kInferRegWarps - 1) / kInferRegWarps));
+    kern<<<grid, kInferRegWarps * 32, smem, st>>>(a);
+    CK(cudaGetLastError());
+}
+
+template <int CH, int STEPS, bool WT>
+inline void launch_infer_reg_g(const InferArgs& a, int num_sms, cudaStream_t st)
+{
+    if (a.pidx || (a.K & 3) || !a.nk_ok || !(a.veta >= 1e-30f && a.veta <= 1e30f))
+        launch_infer_reg_t<CH, 5, WT, true>(a, num_sms, st);
+    else launch_infer_reg_t<CH, STEPS, WT, false>(a, num_sms, st);
+}
+
+template <bool WT>
+inline void launch_infer_reg(const InferArgs& a, int num_sms, cudaStream_t st)
+{
+    if (a.K <= 32) launch_infer_reg_g<1, 3, WT>(a, num_sms, st);
+    else if (a.K <= 64) launch_infer_reg_g<1, 4, WT>(a, num_sms, st);
+    else if (a.K <= 124) launch_infer_reg_g<1, 5, WT>(a, num_sms, st);     // (lane 31 without topics)
+    else if (a.K <= 256) launch_infer_reg_g<2, 5, WT>(a, num_sms, st);
+    else if (a.K <= 384) launch_infer_reg_g<3, 5, WT>(a, num_sms, st);
+    else if (a.K <= 512) launch_infer_reg_g<4, 5, WT>(a, num_sms, st);
+    else launch_infer_reg_g<8, 5, WT>(a, num_sms, st);
 }
 
 // One launch of the slot kernel for this K (the counter must be zeroed first);
 // a.wt != NULL: weighted counts.
 inline void launch_infer(const InferArgs& a, int num_sms, cudaStream_t st)
 {
+    if (a.K <= kInferRegMaxK) {
+        if (a.wt) launch_infer_reg<true>(a, num_sms, st);
+        else launch_infer_reg<false>(a, num_sms, st);
+        return;
+    }
     const uint32_t warps = infer_warps(a.K);
     if (warps == 0) throw ArgError("K too large for on-chip inference state");
     const uint32_t ch = (round4(a.K) + 127) / 128;

@@ -1,0 +1,489 @@
+// infer_reg.cuh -- inference of unseen documents for K <= kInferRegMaxK.
+// Included by infer.cuh inside tmtk, after InferArgs; k_infer_slots there is
+// the kernel of larger K and states the computation.  Both give the same
+// results, bit for bit.
+//
+// What bounds it: a document is one warp's chain of draws (its tokens times its
+// sweeps), so a call lasts as long as its longest documents and the figure that
+// counts is cycles per draw.  Lane l owns topics 128 j + 4 l + i (j < CH); A_k,
+// R_k and the counts sit in shared memory, padded with zeros to 128 CH.  A draw's
+// critical path is the reads of A and R, one fma chain of 4 CH steps, the lane
+// scan's shuffles, the total's broadcast, the choice of a topic and the update
+// of one entry.  Up to CH = 4 every lane forms the prefix sums of its own topics
+// while the scan's shuffles are in flight, so the lane that is hit knows its
+// topic already; above, the hit lane hands its weights to the warp for a second
+// scan (32 prefix sums a lane would cost more than they save).  A and R of
+// the topic that gains the token and of the one that the next token leaves
+// are formed side by side, in different lanes, in one pass.  The next token's column of the frozen
+// n_kw is loaded during the current draw.
+
+constexpr uint32_t kInferRegMaxK = 1024;
+constexpr int kInferRegWarps = 4;    // warps (documents) per block: one per SM sub-partition
+
+//   CH: blocks of four topics per lane (K <= 128 CH); STEPS: steps of the lane scan,
+//       the lanes that hold topics being the first 2^STEPS at most
+//   WT: weighted counts (TermWeight IDF / PMI)
+//   GEN: word priors, K not a multiple of 4 (columns loaded by the element), or
+//       denominators that could leave the range recip needs
+template <int CH, int STEPS, bool WT, bool GEN>
+__global__ void __launch_bounds__(kInferRegWarps * 32, CH <= 2 ? 6 : CH <= 4 ? 4 : 2)
+k_infer_reg(InferArgs a)
+{
+    using CT = typename std::conditional<WT, float, int>::type;
+    using G4 = typename std::conditional<WT, float4, int4>::type;
+    constexpr int T = 4 * CH;
+    constexpr int KW = 128 * CH;
+    constexpr bool kWide = CH > 4;
+    extern __shared__ __align__(16) float s_dyn[];
+    const int K = (int)a.K;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // per block and topic: {n_k (int bits, or float), alpha, eta sum, -}
+    float4* s_st = reinterpret_cast<float4*>(s_dyn);
+    float* s_A = s_dyn + 4 * KW + warp * 4 * KW;
+    float* s_R = s_A + KW;
+    CT* s_n = reinterpret_cast<CT*>(s_R + KW);
+    int* s_own = reinterpret_cast<int*>(s_R + 2 * KW);      // the current run's other tokens per topic
+    // two batches of 32 tokens: {topic | kind << 16, uniform, weight, word}; a draw
+    // leaves its topic in the first.  kind: what follows the token -- 1: the next
+    // one is of the same word (a run goes on); else 3: the next one starts a run;
+    // else 2: a run ends here; else 0
+    __shared__ __align__(16) float4 s_tok_all[kInferRegWarps][64];
+    __shared__ __align__(16) float s_xs_all[kInferRegWarps][kWide ? T : 4];
+    float4* s_tok = s_tok_all[warp];
+    float* s_xs = s_xs_all[warp];
+    const CT* nkw = reinterpret_cast<const CT*>(a.nkw);
+    const CT* nkv = reinterpret_cast<const CT*>(a.nk);
+    CT* ndk_s = reinterpret_cast<CT*>(a.ndk);
+    const unsigned lt = (1u << lane) - 1u;
+    const int left = K - 4 * lane;
+    const int nh = left <= 0 ? 0 : 4 * (left >> 7) + min(left & 127, 4);     // this lane's topics
+    const int last_lane = ((K - 1) >> 2) & 31;                               // the lane of topic K - 1
+    const float eta = a.eta;
+    auto topic_of = [&](int t) { return 128 * (t >> 2) + 4 * lane + (t & 3); };
+    // place of topic k in the per-warp arrays: with CH > 4 block j is turned by j
+    // lanes, so that one lane's topics sit in different banks
+    auto at = [&](int k) { return kWide ? (k & ~127) | ((k + 4 * (k >> 7)) & 127) : k; };
+    const int my4 = 4 * lane;
+    auto blk = [&](int jj) { return 128 * jj + (kWide ? ((my4 + 4 * jj) & 127) : my4); };
+    // Reciprocals, rounded to nearest.  Without priors and with no negative n_k the
+    // denominators lie in [V eta, 2^32 + V eta], and the launch has checked that V eta
+    // lies in [1e-30, 1e30]; one Newton step from an approximation within one ulp is then
+    // exact rounding but for divisors whose mantissa is all ones (P. Markstein,
+    // "Computation of elementary functions on the IBM RISC System/6000
+    // processor", IBM J. Res. Dev. 34, 1990), where it depends on the
+    // approximation: compared with __frcp_rn for every mantissa of the exponents
+    // 2^-107 .. 2^103 on sm_100, no difference.  It has no branch.
+    auto recip = [](float x) -> float {
+        if constexpr (GEN) {
+            return __frcp_rn(x);
+        } else {
+            float y;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+            return __fmaf_rn(y, __fmaf_rn(-x, y, 1.f), y);
+        }
+    };
+    // A and R of a topic with count n (e: its entry)
+    auto eval = [&](const float4& e, CT n, float& A, float& R) {
+        if constexpr (WT) {
+            A = __fadd_rn(n, e.y);
+            R = recip(__fadd_rn(__fadd_rn(e.x, n), e.z));
+        } else {
+            A = __fadd_rn((float)n, e.y);
+            R = recip(__fadd_rn((float)(__float_as_int(e.x) + n), e.z));
+        }
+    };
+    auto less = [&](CT n, float wt) -> CT {     // a token removed
+        if constexpr (WT) return fmaxf(__fsub_rn(n, wt), 0.f);
+        else return n - 1;
+    };
+    auto more = [&](CT n, float wt) -> CT {
+        if constexpr (WT) return __fadd_rn(n, wt);
+        else return n + 1;
+    };
+    for (int k = threadIdx.x; k < KW; k += blockDim.x) {
+        float4 e = make_float4(0.f, 0.f, 1.f, 0.f);
+        if (k < K) {
+            const CT nk = __ldg(nkv + k);
+            if constexpr (WT) e.x = nk;
+            else e.x = __int_as_float(nk);
+            e.y = __ldg(a.alpha + k);
+            e.z = a.esum ? __ldg(a.esum + k) : a.veta;
+        }
+        s_st[k] = e;
+    }
+    for (int k = lane; k < KW; k += 32) {
+        s_A[k] = s_R[k] = 0.f;
+        s_n[k] = CT(0);
+        s_own[k] = 0;
+    }
+    for (int i = lane; i < 64; i += 32) s_tok[i] = make_float4(0.f, 0.f, 0.f, 0.f);   // (read ahead: any word)
+    __syncthreads();
+
+    for (;;) {
+        uint32_t q = 0;
+        if (lane == 0) q = atomicAdd(a.counter, 1u);
+        q = __shfl_sync(FULL, q, 0);
+        if (q >= a.n_work) break;
+        const uint32_t sl = a.work ? a.work[q] : q;
+        const uint64_t b = a.tok_begin[sl];
+        const uint32_t L = a.tok_len ? a.tok_len[sl] : (uint32_t)(a.tok_begin[sl + 1] - b);
+        const uint64_t dk = a.keys ? a.keys[sl] : 0;
+        const uint32_t klo = (uint32_t)dk, khi = (uint32_t)(dk >> 32);
+        const uint32_t it0 = a.it_begin ? a.it_begin[sl] : a.u_begin;
+        const uint32_t it1 = a.it_end ? a.it_end[sl] : a.u_end;
+        const uint32_t itT = a.it_total ? a.it_total[sl] : a.u_total;
+        const uint32_t* words = a.words + b;
+        uint16_t* z = a.z + b;
+        const float* wts = WT ? a.wt + b : nullptr;
+        int nvalid = 0;
+        float wsum = 0.f;                    // WT: the document's weight sum, in token order
+        __syncwarp();
+        if (it0 == 0) {
+            // z0 ~ Discrete(alpha), added to the document's counts
+            for (int k = lane; k < KW; k += 32) s_n[k] = CT(0);
+            __syncwarp();
+            for (uint32_t j = lane; j < L; j += 32) {
+                const uint32_t w = words[j];
+                uint16_t zz = 0xFFFF;
+                if (w < a.V) {
+                    const float u = tmt::u01(tmt::philox_u32(j, 0xFFFFFFFFu, klo, khi, a.key));
+                    const float* cum = a.acum;
+                    if (GEN && a.pidx) {
+                        const int p = a.pidx[w];
+                        cum = p >= 0 ? a.pcum + (uint64_t)p * K : a.ecum;
+                    }
+                    const float r = __fmul_rn(u, cum[K - 1]);
+                    uint32_t lo = 0, hi = K - 1;
+                    while (lo < hi) {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if (r < cum[mid]) hi = mid; else lo = mid + 1;
+                    }
+                    zz = (uint16_t)lo;
+                    if constexpr (!WT) atomicAdd(s_n + at((int)lo), 1);
+                    ++nvalid;
+                }
+                z[j] = zz;
+            }
+            if constexpr (WT) {
+                __syncwarp();
+                if (lane == 0)
+                    for (uint32_t j = 0; j < L; ++j)
+                        if (words[j] < a.V) {
+                            const float wj = wts[j];
+                            CT& n = s_n[at(z[j])];
+                            n = __fadd_rn(n, wj);
+                            wsum = __fadd_rn(wsum, wj);
+                        }
+            }
+        } else {
+            for (int k = lane; k < K; k += 32) s_n[at(k)] = ndk_s[(uint64_t)sl * K + k];
+            for (uint32_t j = lane; j < L; j += 32) nvalid += words[j] < a.V;
+            if (WT && lane == 0)
+                for (uint32_t j = 0; j < L; ++j)
+                    if (words[j] < a.V) wsum = __fadd_rn(wsum, wts[j]);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) nvalid += __shfl_xor_sync(FULL, nvalid, o);
+        if (WT) wsum = __shfl_sync(FULL, wsum, 0);
+        __syncwarp();
+        const uint32_t Lv = (uint32_t)nvalid;    // words are sorted: the sampled tokens come first
+        for (int k = lane; k < K; k += 32) {
+            float A, R;
+            eval(s_st[k], s_n[at(k)], A, R);
+            s_A[at(k)] = A;
+            s_R[at(k)] = R;
+        }
+
+        // a batch's tokens, one per lane, loaded a batch ahead of their staging
+        uint32_t w1 = 0, z1 = 0;
+        float wt1 = 0.f;
+        auto fetch = [&](uint32_t base) {
+            const uint32_t j = base + lane;
+            if (j < Lv) {
+                w1 = words[j];
+                z1 = z[j];
+                if (WT) wt1 = wts[j];
+                const bool same = j + 1 < Lv && words[j + 1] == w1;
+                const bool starts = j + 2 < Lv && words[j + 1] == words[j + 2];
+                const bool ends = j > 0 && words[j - 1] == w1;
+                z1 |= (same ? 1u : starts ? 3u : ends ? 2u : 0u) << 16;
+            }
+        };
+        auto stage = [&](uint32_t base, uint32_t it) {
+            const uint32_t j = base + lane;
+            const float u = tmt::u01(tmt::philox_u32(j, it, klo, khi, a.key));
+            if (j < Lv) s_tok[j & 63] = make_float4(__int_as_float((int)z1), u, wt1, __int_as_float((int)w1));
+        };
+        auto topic = [](const float4& t) { return __float_as_int(t.x) & 0xFFFF; };
+        uint32_t staged = 0;                 // tokens staged so far
+        auto clear_own = [&]() {
+#pragma unroll
+            for (int jj = 0; jj < CH; ++jj) *reinterpret_cast<int4*>(s_own + blk(jj)) = make_int4(0, 0, 0, 0);
+            __syncwarp();
+        };
+        // the run that starts at token j: its other tokens' topics into s_own (zero before)
+        auto start_run = [&](uint32_t j, const float4& t) {
+            for (uint32_t i0 = j;; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                bool in = false;
+                int zi = 0;
+                if (i < staged) {
+                    const float4 e = s_tok[i & 63];
+                    in = __float_as_int(e.w) == __float_as_int(t.w);
+                    zi = topic(e);
+                } else if (i < Lv) {
+                    in = words[i] == (uint32_t)__float_as_int(t.w);
+                    zi = z[i];
+                }
+                if (in && i > j) atomicAdd(&s_own[at(zi)], 1);
+                if (__ballot_sync(FULL, !in)) break;
+            }
+            __syncwarp();
+        };
+        auto load_col = [&](float word, G4 (&g)[CH]) {
+            const CT* col = nkw + (uint64_t)(uint32_t)__float_as_int(word) * (uint32_t)K + my4;
+#pragma unroll
+            for (int jj = 0; jj < CH; ++jj) {
+                const int k0 = 128 * jj + my4;
+                g[jj].x = g[jj].y = g[jj].z = g[jj].w = CT(0);
+                if constexpr (!GEN) {
+                    if (k0 < K) g[jj] = __ldg(reinterpret_cast<const G4*>(col + 128 * jj));
+                } else {
+                    if (k0 < K) g[jj].x = __ldg(col + 128 * jj);
+                    if (k0 + 1 < K) g[jj].y = __ldg(col + 128 * jj + 1);
+                    if (k0 + 2 < K) g[jj].z = __ldg(col + 128 * jj + 2);
+                    if (k0 + 3 < K) g[jj].w = __ldg(col + 128 * jj + 3);
+                }
+            }
+        };
+
+        for (uint32_t it = it0; it < it1 && Lv; ++it) {
+            fetch(0);
+            stage(0, it);
+            staged = min(32u, Lv);
+            fetch(32);
+            __syncwarp();
+            float4 tok = s_tok[0];
+            G4 g[CH];
+            load_col(tok.w, g);
+            {
+                // the first token leaves its topic
+                const int zo = topic(tok);
+                const CT n = less(s_n[at(zo)], tok.z);
+                float A, R;
+                eval(s_st[zo], n, A, R);
+                __syncwarp();
+                if (lane == 0) {
+                    s_n[at(zo)] = n;
+                    s_A[at(zo)] = A;
+                    s_R[at(zo)] = R;
+                }
+                __syncwarp();
+                if ((__float_as_int(tok.x) >> 16) == 1) start_run(0, tok);
+            }
+            for (uint32_t base = 0; base < Lv; base += 32) {
+              if (staged < Lv) {
+                  // the next batch's tokens into the other half of the ring; the one
+                  // after it on its way
+                  stage(staged, it);
+                  staged = min(staged + 32, Lv);
+                  fetch(staged);
+                  __syncwarp();
+              }
+              const uint32_t end = min(base + 32, Lv);
+#pragma unroll 1
+              for (uint32_t jt = base; jt < end; ++jt) {
+                const float4 nt = s_tok[(jt + 1) & 63];
+                G4 gn[CH];
+                load_col(nt.w, gn);
+                const bool more_tokens = jt + 1 < Lv;
+                const int zn = topic(nt);            // the topic the next token leaves (if there is one)
+                const int kind = __float_as_int(tok.x) >> 16;
+                const float u = tok.y, wt = tok.z;
+                // the run's other tokens of the word (zero outside a run)
+#pragma unroll
+                for (int jj = 0; jj < CH; ++jj) {
+                    const int4 o = *reinterpret_cast<const int4*>(s_own + blk(jj));
+                    if constexpr (WT) {
+                        g[jj].x = __fadd_rn(g[jj].x, __fmul_rn((float)o.x, wt));
+                        g[jj].y = __fadd_rn(g[jj].y, __fmul_rn((float)o.y, wt));
+                        g[jj].z = __fadd_rn(g[jj].z, __fmul_rn((float)o.z, wt));
+                        g[jj].w = __fadd_rn(g[jj].w, __fmul_rn((float)o.w, wt));
+                    } else {
+                        g[jj].x += o.x;
+                        g[jj].y += o.y;
+                        g[jj].z += o.z;
+                        g[jj].w += o.w;
+                    }
+                }
+                const float* pe = nullptr;           // the word's prior column, if any
+                if (GEN && a.pidx) {
+                    const int p = __ldg(a.pidx + (uint32_t)__float_as_int(tok.w));
+                    if (p >= 0) pe = a.pval + (uint64_t)p * K;
+                }
+                auto ek = [&](int t) { return GEN && pe && topic_of(t) < K ? __ldg(pe + topic_of(t)) : eta; };
+                // pass 1: fma chain over this lane's topics; w: A_k for CH <= 4
+                // turned into the weights, above B_k R_k
+                float w[T], s = 0.f;
+#pragma unroll
+                for (int jj = 0; jj < CH; ++jj) {
+                    const float4 A4 = *reinterpret_cast<const float4*>(s_A + blk(jj));
+                    const float4 R4 = *reinterpret_cast<const float4*>(s_R + blk(jj));
+                    w[4 * jj] = __fmul_rn(__fadd_rn((float)g[jj].x, ek(4 * jj)), R4.x);
+                    w[4 * jj + 1] = __fmul_rn(__fadd_rn((float)g[jj].y, ek(4 * jj + 1)), R4.y);
+                    w[4 * jj + 2] = __fmul_rn(__fadd_rn((float)g[jj].z, ek(4 * jj + 2)), R4.z);
+                    w[4 * jj + 3] = __fmul_rn(__fadd_rn((float)g[jj].w, ek(4 * jj + 3)), R4.w);
+                    s = __fmaf_rn(A4.x, w[4 * jj], s);
+                    s = __fmaf_rn(A4.y, w[4 * jj + 1], s);
+                    s = __fmaf_rn(A4.z, w[4 * jj + 2], s);
+                    s = __fmaf_rn(A4.w, w[4 * jj + 3], s);
+                    if constexpr (!kWide) {
+                        w[4 * jj] = __fmul_rn(A4.x, w[4 * jj]);
+                        w[4 * jj + 1] = __fmul_rn(A4.y, w[4 * jj + 1]);
+                        w[4 * jj + 2] = __fmul_rn(A4.z, w[4 * jj + 2]);
+                        w[4 * jj + 3] = __fmul_rn(A4.w, w[4 * jj + 3]);
+                    }
+                }
+                float x = s;
+#pragma unroll
+                for (int i = 0; i < STEPS; ++i) x = hs_up(x, 1 << i);
+                const float total = __shfl_sync(FULL, x, (1 << STEPS) - 1);
+                const float E = up1_or_0(x);
+                const float r = __fmul_rn(u, total);
+                const bool in = nh > 0 && r < __fadd_rn(E, s);
+                int knew = 0;                        // the new topic (in the lane that keeps it)
+                bool keep;
+                if constexpr (!kWide) {
+                    // prefix sums of this lane's own weights (Hillis-Steele order)
+#pragma unroll
+                    for (int off = 1; off < T; off <<= 1) {
+#pragma unroll
+                        for (int t = T - 1; t >= off; --t) w[t] = __fadd_rn(w[t], w[t - off]);
+                    }
+                    int found = T - 1;
+#pragma unroll
+                    for (int t = T - 2; t >= 0; --t)
+                        if (r < __fadd_rn(E, w[t])) found = t;
+                    found = in ? min(found, nh - 1) : max(nh - 1, 0);
+                    knew = topic_of(found);
+                    // One lane forms the next token's removal (lane 31, which holds no
+                    // topic, with CH = 1, else the lane of that topic), every other lane
+                    // the addition to the topic it would draw.
+                    const bool mine = more_tokens && lane == (CH == 1 ? 31 : (zn >> 2) & 31);
+                    const int kx = mine ? zn : knew;
+                    const CT n = s_n[kx];
+                    CT nx = mine ? less(n, nt.z) : more(n, wt);
+                    // (the addition to the topic that the next token leaves)
+                    if (CH == 1 && more_tokens && !mine && knew == zn) nx = less(nx, nt.z);
+                    float Ax, Rx;
+                    eval(s_st[kx], nx, Ax, Rx);
+                    // the first lane that r falls in; topic K - 1 when rounding left it
+                    // at or above the total
+                    unsigned m = __ballot_sync(FULL, in);
+                    if (m == 0) m = 1u << last_lane;
+                    const bool hit = (m & (0u - m)) == lt + 1u;
+                    keep = hit;
+                    __syncwarp();                    // every lane has read its entries
+                    if constexpr (CH == 1) {
+                        // the removal first: an addition to the same topic overwrites it
+                        if (mine) {
+                            s_n[kx] = nx;
+                            s_A[kx] = Ax;
+                            s_R[kx] = Rx;
+                        }
+                        __syncwarp();
+                        if (hit) {
+                            s_n[kx] = nx;
+                            s_A[kx] = Ax;
+                            s_R[kx] = Rx;
+                        }
+                    } else {
+                        if (hit && mine) {           // both in this lane
+                            CT n2 = more(s_n[knew], wt);
+                            if (knew == zn) n2 = less(n2, nt.z);
+                            float A2, R2;
+                            eval(s_st[knew], n2, A2, R2);
+                            if (knew == zn) {
+                                nx = n2;
+                                Ax = A2;
+                                Rx = R2;
+                            } else {
+                                s_n[knew] = n2;
+                                s_A[knew] = A2;
+                                s_R[knew] = R2;
+                            }
+                        }
+                        if (hit || mine) {
+                            s_n[kx] = nx;
+                            s_A[kx] = Ax;
+                            s_R[kx] = Rx;
+                        }
+                    }
+                } else {
+                    const unsigned m = __ballot_sync(FULL, in);
+                    knew = K - 1;
+                    if (m) {
+                        // pass 2: position among lane h's topics
+                        const int h = __ffs(m) - 1;
+                        const float Eh = __shfl_sync(FULL, E, h);
+                        if (lane == h) {
+#pragma unroll
+                            for (int jj = 0; jj < CH; ++jj)
+                                *reinterpret_cast<float4*>(s_xs + 4 * jj) =
+                                    make_float4(w[4 * jj], w[4 * jj + 1], w[4 * jj + 2], w[4 * jj + 3]);
+                        }
+                        const int mh = K - 4 * h;
+                        const int nhh = 4 * (mh >> 7) + min(mh & 127, 4);
+                        const int k = 128 * (lane >> 2) + 4 * h + (lane & 3);
+                        __syncwarp();
+                        float x2 = 0.f;
+                        if (lane < nhh) x2 = __fmul_rn(s_A[at(k)], s_xs[lane]);
+#pragma unroll
+                        for (int i = 0; i < 5; ++i) x2 = hs_up(x2, 1 << i);
+                        const unsigned mb = __ballot_sync(FULL, lane < nhh && r < __fadd_rn(Eh, x2));
+                        const int found = mb ? __ffs(mb) - 1 : nhh - 1;
+                        knew = 128 * (found >> 2) + 4 * h + (found & 3);
+                    }
+                    // lane 0 forms the addition, lane 1 the next token's removal
+                    const bool both = more_tokens && knew == zn;
+                    const int kx = lane == 1 && more_tokens ? zn : knew;
+                    const CT n = s_n[at(kx)];
+                    CT nx = lane == 1 ? less(n, nt.z) : more(n, wt);
+                    if (both) nx = less(more(n, wt), nt.z);
+                    float Ax, Rx;
+                    eval(s_st[kx], nx, Ax, Rx);
+                    keep = lane == 0;
+                    __syncwarp();                    // every lane has read its entries
+                    if (lane == 0 || (lane == 1 && more_tokens && !both)) {
+                        s_n[at(kx)] = nx;
+                        s_A[at(kx)] = Ax;
+                        s_R[at(kx)] = Rx;
+                    }
+                }
+                if (keep) s_tok[jt & 63].x = __int_as_float(knew);
+                if (kind) {
+                    if (kind == 1) {
+                        if (keep) atomicAdd(&s_own[at(knew)], 1);
+                        if (lane == 0) atomicSub(&s_own[at(zn)], 1);
+                    } else {
+                        clear_own();
+                        if (kind == 3) start_run(jt + 1, nt);
+                    }
+                }
+                __syncwarp();
+                tok = nt;
+#pragma unroll
+                for (int jj = 0; jj < CH; ++jj) g[jj] = gn[jj];
+              }
+              if (base + lane < end) z[base + lane] = (uint16_t)__float_as_int(s_tok[(base + lane) & 63].x);
+              __syncwarp();
+            }
+        }
+        if (it1 < itT) {            // keep the document's counts for the next launch
+            for (int k = lane; k < K; k += 32) ndk_s[(uint64_t)sl * K + k] = s_n[at(k)];
+            continue;
+        }
+        // finished: theta, FP64 ll over the touched cells
+        finish_doc<WT>(a, sl, b, L, WT ? wsum : (float)nvalid, lane, s_own, [&](int k) -> CT { return s_n[at(k)]; });
+    }
+}

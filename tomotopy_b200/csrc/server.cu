@@ -167,6 +167,7 @@ struct Model {
     float* d_pcum = nullptr;
     float* d_ecum = nullptr;
     bool used = false;                  // a request was submitted: the model is frozen
+    bool nk_ok = true;                  // no negative n_k
     bool weighted = false;              // float counts (TermWeight IDF / PMI); requests carry weights
 };
 
@@ -394,6 +395,7 @@ bool server_step(tmt_server* s)
         a.esum = m->d_esum;
         a.pcum = m->d_pcum;
         a.ecum = m->d_ecum;
+        a.nk_ok = m->nk_ok;
         // every request of a model shares the draw key base; the per-request seed is folded in below
         a.key = 0;
         // requests may carry different seeds: launch per distinct seed (usually one)
@@ -578,6 +580,9 @@ tmt_status add_model_impl(tmt_server* s, uint32_t K, uint32_t V, const float* al
     m->asum_f = sf;
     m->asum_d = sd;
     m->weighted = weighted;
+    for (uint32_t k = 0; k < K && n_k; ++k)
+        if (!(weighted ? static_cast<const float*>(n_k)[k] >= 0.f : static_cast<const int32_t*>(n_k)[k] >= 0))
+            m->nk_ok = false;
     const uint32_t S = s->cfg.max_slots;
     m->slots = S;
     m->active.assign(S, -1);
