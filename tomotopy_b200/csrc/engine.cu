@@ -1316,7 +1316,9 @@ struct tmt_handle {
     double* d_llv = nullptr;         // tmt_ll output (2)
     double* d_partials = nullptr;
     uint32_t n_partials = 0;
-    bool nk_ok = true;               // no negative n_k (set_counts may bring some)
+    // counts set from outside (set_counts): the largest of n_kw (2^32 - 1: some may be
+    // negative); else n_kw is bounded by n_k
+    uint64_t set_max = 0;
     double* d_ll = nullptr;          // ll history for one train() call (2 per point)
     uint32_t ll_cap = 0;
     float* d_dg_points = nullptr;
@@ -2200,7 +2202,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
         }
         h->release();
         h->uploaded = false;
-        h->nk_ok = true;
+        h->set_max = 0;
         h->D = D;
         h->N_all = n_all;
         h->global_step = 0;
@@ -2697,7 +2699,13 @@ tmt_status tmt_set_counts(tmt_handle* h, const int32_t* n_kw, const int32_t* n_k
         const uint64_t kv = (uint64_t)h->cfg.K * h->cfg.V;
         h2d(h, h->d_nkw[h->cur], n_kw, kv * sizeof(int32_t));
         CK(cudaMemcpyAsync(h->d_nk[h->cur], n_k, h->cfg.K * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
-        h->nk_ok = *std::min_element(n_k, n_k + h->cfg.K) >= 0;
+        CK(cudaMemsetAsync(h->d_counter, 0, sizeof(uint32_t), h->stream));
+        k_max_count<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_nkw[h->cur], kv, h->d_counter);
+        launch_check(h);
+        uint32_t mx = 0;
+        CK(cudaMemcpyAsync(&mx, h->d_counter, sizeof(mx), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        h->set_max = std::max<uint64_t>(1, mx);
         CK(cudaStreamSynchronize(h->stream));
     });
 }
@@ -3063,7 +3071,14 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         }
         // alpha of the current state (after any optimisation)
         CK(cudaMemcpyAsync(h->alpha.data(), h->d_alpha, K * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        std::vector<int32_t> nk(K);                // (float bits when weighted)
+        CK(cudaMemcpyAsync(nk.data(), h->d_nk[h->cur], K * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
+        // the largest count with a document's tokens added (integer counts; after
+        // set_counts training may have moved up to N tokens onto a cell)
+        uint64_t longest = 0, most = h->set_max ? h->set_max + h->N : 0;
+        for (uint64_t d = 0; d < D; ++d) longest = std::max(longest, doc_off[d + 1] - doc_off[d]);
+        for (uint32_t k = 0; k < K; ++k) most = std::max<uint64_t>(most, (uint32_t)nk[k]);
         std::vector<float> acum(K);
         float sf = 0.f;
         double sd = 0;
@@ -3119,7 +3134,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         a.esum = h->d_esum;
         a.pcum = h->d_prior_cum;
         a.ecum = h->d_cum_eta;
-        a.nk_ok = h->nk_ok;
+        a.small_counts = h->weighted || most + longest < (1u << 23);   // (weighted counts are never negative)
         launch_infer(a, h->num_sms, h->stream);
         ++h->launches;
         if (theta) d2h(h, theta, B.theta, D * (uint64_t)K * sizeof(float));

@@ -65,8 +65,9 @@ struct InferArgs {
     const float* esum;
     const float* pcum;
     const float* ecum;
-    // the caller's n_k holds no negative value (only counts set from outside can)
-    bool nk_ok;
+    // no n_k (nor n_kw) is negative, and with a document's tokens added none
+    // reaches 2^23 (weighted counts: only the former)
+    bool small_counts;
 };
 
 // A finished document's theta and FP64 ll over the cells it touched.  dlen: its
@@ -465,11 +466,11 @@ inline void launch_infer_w(const InferArgs& a, uint32_t warps, uint32_t ch, int 
     else launch_infer_t<0, WT>(a, warps, num_sms, st);
 }
 
-template <int CH, int STEPS, bool WT, bool GEN>
+template <int CH, int STEPS, bool WT, int MODE>
 inline void launch_infer_reg_t(const InferArgs& a, int num_sms, cudaStream_t st)
 {
-    auto kern = k_infer_reg<CH, STEPS, WT, GEN>;
-    const uint32_t smem = (kInferRegWarps + 1) * 16 * 128 * CH;
+    auto kern = k_infer_reg<CH, STEPS, WT, MODE>;
+    const uint32_t smem = (4 + kInferRegWarps * (!WT && CH <= 4 ? 6 : 4)) * 4 * 128 * CH;     // (k_infer_reg's s_dyn)
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kInferRegWarps * 32, smem));
@@ -483,9 +484,16 @@ inline void launch_infer_reg_t(const InferArgs& a, int num_sms, cudaStream_t st)
 template <int CH, int STEPS, bool WT>
 inline void launch_infer_reg_g(const InferArgs& a, int num_sms, cudaStream_t st)
 {
-    if (a.pidx || (a.K & 3) || !a.nk_ok || !(a.veta >= 1e-30f && a.veta <= 1e30f))
-        launch_infer_reg_t<CH, 5, WT, true>(a, num_sms, st);
-    else launch_infer_reg_t<CH, STEPS, WT, false>(a, num_sms, st);
+    // The fast modes' conditions: scalar eta, counts exact in to_f, denominators in
+    // recip's range.  (Their general forms cost a draw at k = 100 about 50 of 450
+    // cycles.)  Element loads where columns are not 16-byte aligned.
+    // (No weight or sum of weights can overflow: A B R below 1e36 / K.)
+    const double most = WT ? 549755813888.0 : 8388608.0;
+    const bool finite = (most + (double)a.asum_f) * (most + (double)a.eta) < 1e32 * (double)a.veta;
+    if (a.pidx || !a.small_counts || !finite || !(a.veta >= 1e-30f && a.veta <= 1e30f))
+        launch_infer_reg_t<CH, 5, WT, 2>(a, num_sms, st);
+    else if (a.K & 3) launch_infer_reg_t<CH, STEPS, WT, 1>(a, num_sms, st);
+    else launch_infer_reg_t<CH, STEPS, WT, 0>(a, num_sms, st);
 }
 
 template <bool WT>
@@ -498,6 +506,16 @@ inline void launch_infer_reg(const InferArgs& a, int num_sms, cudaStream_t st)
     else if (a.K <= 384) launch_infer_reg_g<3, 5, WT>(a, num_sms, st);
     else if (a.K <= 512) launch_infer_reg_g<4, 5, WT>(a, num_sms, st);
     else launch_infer_reg_g<8, 5, WT>(a, num_sms, st);
+}
+
+// the largest of n counts, negative ones as large (out must be 0 before)
+static __global__ void k_max_count(const int32_t* __restrict__ c, uint64_t n, uint32_t* __restrict__ out)
+{
+    uint32_t m = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        m = max(m, (uint32_t)c[i]);
+    m = __reduce_max_sync(FULL, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
 // One launch of the slot kernel for this K (the counter must be zeroed first);

@@ -23,28 +23,38 @@ constexpr int kInferRegWarps = 4;    // warps (documents) per block: one per SM 
 //   CH: blocks of four topics per lane (K <= 128 CH); STEPS: steps of the lane scan,
 //       the lanes that hold topics being the first 2^STEPS at most
 //   WT: weighted counts (TermWeight IDF / PMI)
-//   GEN: word priors, K not a multiple of 4 (columns loaded by the element), or
-//       denominators that could leave the range recip needs
-template <int CH, int STEPS, bool WT, bool GEN>
-__global__ void __launch_bounds__(kInferRegWarps * 32, CH <= 2 ? 6 : CH <= 4 ? 4 : 2)
+//   MODE 0: K a multiple of 4 and the launch's fast conditions (launch_infer_reg_g);
+//        1: the fast conditions, columns loaded by the element;
+//        2: any (word priors, counts of 2^23 and more, extreme V eta)
+template <int CH, int STEPS, bool WT, int MODE>
+__global__ void __launch_bounds__(kInferRegWarps * 32, CH <= 1 ? 5 : CH <= 2 ? 6 : CH <= 4 ? 4 : 2)
 k_infer_reg(InferArgs a)
 {
     using CT = typename std::conditional<WT, float, int>::type;
     using G4 = typename std::conditional<WT, float4, int4>::type;
     constexpr int T = 4 * CH;
     constexpr int KW = 128 * CH;
+    constexpr bool GEN = MODE == 2;
     constexpr bool kWide = CH > 4;
+    // integer counts up to CH = 4: A and R of one token more are kept for every topic
+    constexpr bool kPlus = !WT && !kWide;
+    constexpr int kArrays = kPlus ? 6 : 4;
     extern __shared__ __align__(16) float s_dyn[];
     const int K = (int)a.K;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // per block and topic: {n_k (int bits, or float), alpha, eta sum, -}
     float4* s_st = reinterpret_cast<float4*>(s_dyn);
-    float* s_A = s_dyn + 4 * KW + warp * 4 * KW;
+    // per warp: A, R, counts, the current run's other tokens per topic and, with
+    // kPlus, A and R of one token more -- kArrays arrays of KW words, one address with offsets
+    float* s_A = s_dyn + 4 * KW + warp * kArrays * KW;
     float* s_R = s_A + KW;
-    CT* s_n = reinterpret_cast<CT*>(s_R + KW);
-    int* s_own = reinterpret_cast<int*>(s_R + 2 * KW);      // the current run's other tokens per topic
-    // two batches of 32 tokens: {topic | kind << 16, uniform, weight, word}; a draw
-    // leaves its topic in the first.  kind: what follows the token -- 1: the next
+    CT* s_n = reinterpret_cast<CT*>(s_A + 2 * KW);
+    int* s_own = reinterpret_cast<int*>(s_A + 3 * KW);
+    float* s_Ap = s_A + (kPlus ? 4 : 0) * KW;
+    float* s_Rp = s_A + (kPlus ? 5 : 0) * KW;
+    // two batches of 32 tokens: {topic | kind << 16 | run << 18, uniform, weight,
+    // word}; a draw leaves its topic in the first.  run: the tokens of its word from
+    // it on, 0 when they go on past the batch.  kind: what follows the token -- 1: the next
     // one is of the same word (a run goes on); else 3: the next one starts a run;
     // else 2: a run ends here; else 0
     __shared__ __align__(16) float4 s_tok_all[kInferRegWarps][64];
@@ -65,9 +75,9 @@ k_infer_reg(InferArgs a)
     auto at = [&](int k) { return kWide ? (k & ~127) | ((k + 4 * (k >> 7)) & 127) : k; };
     const int my4 = 4 * lane;
     auto blk = [&](int jj) { return 128 * jj + (kWide ? ((my4 + 4 * jj) & 127) : my4); };
-    // Reciprocals, rounded to nearest.  Without priors and with no negative n_k the
-    // denominators lie in [V eta, 2^32 + V eta], and the launch has checked that V eta
-    // lies in [1e-30, 1e30]; one Newton step from an approximation within one ulp is then
+    // Reciprocals, rounded to nearest.  In the fast modes the denominators lie in
+    // [V eta, 2^23 + V eta] (weighted: n_k's range above V eta) with V eta in [1e-30,
+    // 1e30]; one Newton step from an approximation within one ulp is then
     // exact rounding but for divisors whose mantissa is all ones (P. Markstein,
     // "Computation of elementary functions on the IBM RISC System/6000
     // processor", IBM J. Res. Dev. 34, 1990), where it depends on the
@@ -82,14 +92,20 @@ k_infer_reg(InferArgs a)
             return __fmaf_rn(y, __fmaf_rn(-x, y, 1.f), y);
         }
     };
+    // (float)n of a count: in the fast modes below 2^23, where 2^23 + n is exact in
+    // the float whose mantissa holds n (the conversion unit does one warp in 8 cycles)
+    auto to_f = [](CT n) -> float {
+        if constexpr (WT || GEN) return (float)n;
+        else return __fsub_rn(__int_as_float(n | 0x4B000000), 8388608.f);
+    };
     // A and R of a topic with count n (e: its entry)
     auto eval = [&](const float4& e, CT n, float& A, float& R) {
         if constexpr (WT) {
             A = __fadd_rn(n, e.y);
             R = recip(__fadd_rn(__fadd_rn(e.x, n), e.z));
         } else {
-            A = __fadd_rn((float)n, e.y);
-            R = recip(__fadd_rn((float)(__float_as_int(e.x) + n), e.z));
+            A = __fadd_rn(to_f(n), e.y);
+            R = recip(__fadd_rn(to_f(__float_as_int(e.x) + n), e.z));
         }
     };
     auto less = [&](CT n, float wt) -> CT {     // a token removed
@@ -99,6 +115,14 @@ k_infer_reg(InferArgs a)
     auto more = [&](CT n, float wt) -> CT {
         if constexpr (WT) return __fadd_rn(n, wt);
         else return n + 1;
+    };
+    float lm[5];                             // 1 in the lanes at or above 2^i, else 0
+#pragma unroll
+    for (int i = 0; i < 5; ++i) lm[i] = lane >= (1 << i) ? 1.f : 0.f;
+    // a scan step: for finite sums fma(y, 1, x) rounds as x + y and fma(y, 0, x) is x
+    auto scan_step = [&](float x, int i) {
+        if constexpr (GEN) return hs_up(x, 1 << i);
+        else return __fmaf_rn(__shfl_up_sync(FULL, x, 1 << i), lm[i], x);
     };
     for (int k = threadIdx.x; k < KW; k += blockDim.x) {
         float4 e = make_float4(0.f, 0.f, 1.f, 0.f);
@@ -118,6 +142,33 @@ k_infer_reg(InferArgs a)
     }
     for (int i = lane; i < 64; i += 32) s_tok[i] = make_float4(0.f, 0.f, 0.f, 0.f);   // (read ahead: any word)
     __syncthreads();
+
+    // predicated stores (a store under `if` is a branch on every draw's chain):
+    // count, A and R of a topic ...
+    auto put = [](bool p, float* at_a, CT n, float A, float R) {
+        float nb;
+        if constexpr (WT) nb = n;
+        else nb = __int_as_float(n);
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p st.shared.f32 [%1], %3;\n"
+                     " @p st.shared.f32 [%1+%5], %4;\n @p st.shared.f32 [%1+%6], %2;\n}"
+                     :: "r"((int)p), "r"((uint32_t)__cvta_generic_to_shared(at_a)), "f"(nb), "f"(A), "f"(R),
+                        "n"(4 * KW), "n"(8 * KW) : "memory");
+    };
+    // ... and its A and R of one token more
+    auto put_plus = [](bool p, float* at_a, float A, float R) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p st.shared.f32 [%1+%4], %2;\n"
+                     " @p st.shared.f32 [%1+%5], %3;\n}"
+                     :: "r"((int)p), "r"((uint32_t)__cvta_generic_to_shared(at_a)), "f"(A), "f"(R),
+                        "n"(16 * KW), "n"(20 * KW) : "memory");
+    };
+    auto put_i = [](bool p, void* at, int v) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p st.shared.s32 [%1], %2;\n}"
+                     :: "r"((int)p), "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(v) : "memory");
+    };
+    auto add_own = [](bool p, float* at_a, int v) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p red.shared.add.s32 [%1+%3], %2;\n}"
+                     :: "r"((int)p), "r"((uint32_t)__cvta_generic_to_shared(at_a)), "r"(v), "n"(12 * KW) : "memory");
+    };
 
     for (;;) {
         uint32_t q = 0;
@@ -192,6 +243,11 @@ k_infer_reg(InferArgs a)
             eval(s_st[k], s_n[at(k)], A, R);
             s_A[at(k)] = A;
             s_R[at(k)] = R;
+            if constexpr (kPlus) {
+                eval(s_st[k], more(s_n[k], 0.f), A, R);
+                s_Ap[k] = A;
+                s_Rp[k] = R;
+            }
         }
 
         // a batch's tokens, one per lane, loaded a batch ahead of their staging
@@ -208,6 +264,8 @@ k_infer_reg(InferArgs a)
                 const bool ends = j > 0 && words[j - 1] == w1;
                 z1 |= (same ? 1u : starts ? 3u : ends ? 2u : 0u) << 16;
             }
+            const unsigned stops = __ballot_sync(FULL, j >= Lv || ((z1 >> 16) & 3) != 1) >> lane;
+            if (j < Lv) z1 |= (uint32_t)__ffs(stops) << 18;
         };
         auto stage = [&](uint32_t base, uint32_t it) {
             const uint32_t j = base + lane;
@@ -215,6 +273,7 @@ k_infer_reg(InferArgs a)
             if (j < Lv) s_tok[j & 63] = make_float4(__int_as_float((int)z1), u, wt1, __int_as_float((int)w1));
         };
         auto topic = [](const float4& t) { return __float_as_int(t.x) & 0xFFFF; };
+        auto kind_of = [](const float4& t) { return (__float_as_int(t.x) >> 16) & 3; };
         uint32_t staged = 0;                 // tokens staged so far
         auto clear_own = [&]() {
 #pragma unroll
@@ -223,6 +282,12 @@ k_infer_reg(InferArgs a)
         };
         // the run that starts at token j: its other tokens' topics into s_own (zero before)
         auto start_run = [&](uint32_t j, const float4& t) {
+            if (const int run = __float_as_int(t.x) >> 18) {
+                const int zi = topic(s_tok[(j + 1 + lane) & 63]);
+                add_own(lane < run - 1, s_A + at(min(zi, K - 1)), 1);
+                __syncwarp();
+                return;
+            }
             for (uint32_t i0 = j;; i0 += 32) {
                 const uint32_t i = i0 + lane;
                 bool in = false;
@@ -240,13 +305,13 @@ k_infer_reg(InferArgs a)
             }
             __syncwarp();
         };
+        // (a lane's blocks past K are never loaded and stay 0)
         auto load_col = [&](float word, G4 (&g)[CH]) {
             const CT* col = nkw + (uint64_t)(uint32_t)__float_as_int(word) * (uint32_t)K + my4;
 #pragma unroll
             for (int jj = 0; jj < CH; ++jj) {
                 const int k0 = 128 * jj + my4;
-                g[jj].x = g[jj].y = g[jj].z = g[jj].w = CT(0);
-                if constexpr (!GEN) {
+                if constexpr (MODE == 0) {
                     if (k0 < K) g[jj] = __ldg(reinterpret_cast<const G4*>(col + 128 * jj));
                 } else {
                     if (k0 < K) g[jj].x = __ldg(col + 128 * jj);
@@ -257,6 +322,7 @@ k_infer_reg(InferArgs a)
             }
         };
 
+        int kp = -1;                         // kPlus: the topic this lane last added to, its plus entry not yet renewed
         for (uint32_t it = it0; it < it1 && Lv; ++it) {
             fetch(0);
             stage(0, it);
@@ -264,22 +330,26 @@ k_infer_reg(InferArgs a)
             fetch(32);
             __syncwarp();
             float4 tok = s_tok[0];
-            G4 g[CH];
-            load_col(tok.w, g);
+            G4 ga[CH], gb[CH];               // the columns of even and odd tokens
+#pragma unroll
+            for (int jj = 0; jj < CH; ++jj) {
+                ga[jj].x = ga[jj].y = ga[jj].z = ga[jj].w = CT(0);
+                gb[jj] = ga[jj];
+            }
+            load_col(tok.w, ga);
+            bool in_run = kind_of(tok) == 1;
             {
                 // the first token leaves its topic
                 const int zo = topic(tok);
                 const CT n = less(s_n[at(zo)], tok.z);
                 float A, R;
                 eval(s_st[zo], n, A, R);
+                const float A0 = s_A[at(zo)], R0 = s_R[at(zo)];
                 __syncwarp();
-                if (lane == 0) {
-                    s_n[at(zo)] = n;
-                    s_A[at(zo)] = A;
-                    s_R[at(zo)] = R;
-                }
+                put(lane == 0, s_A + at(zo), n, A, R);
+                if constexpr (kPlus) put_plus(lane == 0, s_A + zo, A0, R0);
                 __syncwarp();
-                if ((__float_as_int(tok.x) >> 16) == 1) start_run(0, tok);
+                if (in_run) start_run(0, tok);
             }
             for (uint32_t base = 0; base < Lv; base += 32) {
               if (staged < Lv) {
@@ -291,16 +361,16 @@ k_infer_reg(InferArgs a)
                   __syncwarp();
               }
               const uint32_t end = min(base + 32, Lv);
-#pragma unroll 1
-              for (uint32_t jt = base; jt < end; ++jt) {
+              // one token: its column in g, the next one's into gn
+              auto step = [&](uint32_t jt, G4 (&g)[CH], G4 (&gn)[CH]) {
                 const float4 nt = s_tok[(jt + 1) & 63];
-                G4 gn[CH];
                 load_col(nt.w, gn);
                 const bool more_tokens = jt + 1 < Lv;
-                const int zn = topic(nt);            // the topic the next token leaves (if there is one)
-                const int kind = __float_as_int(tok.x) >> 16;
+                const int zn = min(topic(nt), K - 1);    // the topic the next token leaves (if there is one)
+                const int kind = kind_of(tok);
                 const float u = tok.y, wt = tok.z;
                 // the run's other tokens of the word (zero outside a run)
+                if (CH <= 2 || in_run)
 #pragma unroll
                 for (int jj = 0; jj < CH; ++jj) {
                     const int4 o = *reinterpret_cast<const int4*>(s_own + blk(jj));
@@ -329,10 +399,10 @@ k_infer_reg(InferArgs a)
                 for (int jj = 0; jj < CH; ++jj) {
                     const float4 A4 = *reinterpret_cast<const float4*>(s_A + blk(jj));
                     const float4 R4 = *reinterpret_cast<const float4*>(s_R + blk(jj));
-                    w[4 * jj] = __fmul_rn(__fadd_rn((float)g[jj].x, ek(4 * jj)), R4.x);
-                    w[4 * jj + 1] = __fmul_rn(__fadd_rn((float)g[jj].y, ek(4 * jj + 1)), R4.y);
-                    w[4 * jj + 2] = __fmul_rn(__fadd_rn((float)g[jj].z, ek(4 * jj + 2)), R4.z);
-                    w[4 * jj + 3] = __fmul_rn(__fadd_rn((float)g[jj].w, ek(4 * jj + 3)), R4.w);
+                    w[4 * jj] = __fmul_rn(__fadd_rn(to_f(g[jj].x), ek(4 * jj)), R4.x);
+                    w[4 * jj + 1] = __fmul_rn(__fadd_rn(to_f(g[jj].y), ek(4 * jj + 1)), R4.y);
+                    w[4 * jj + 2] = __fmul_rn(__fadd_rn(to_f(g[jj].z), ek(4 * jj + 2)), R4.z);
+                    w[4 * jj + 3] = __fmul_rn(__fadd_rn(to_f(g[jj].w), ek(4 * jj + 3)), R4.w);
                     s = __fmaf_rn(A4.x, w[4 * jj], s);
                     s = __fmaf_rn(A4.y, w[4 * jj + 1], s);
                     s = __fmaf_rn(A4.z, w[4 * jj + 2], s);
@@ -346,9 +416,25 @@ k_infer_reg(InferArgs a)
                 }
                 float x = s;
 #pragma unroll
-                for (int i = 0; i < STEPS; ++i) x = hs_up(x, 1 << i);
+                for (int i = 0; i < STEPS; ++i) x = scan_step(x, i);
                 const float total = __shfl_sync(FULL, x, (1 << STEPS) - 1);
-                const float E = up1_or_0(x);
+                const float E = GEN ? up1_or_0(x) : __fmul_rn(__shfl_up_sync(FULL, x, 1), lm[0]);
+                // the next token's removal, should this draw leave its topic alone
+                float Az = 0.f, Rz = 0.f, Az0 = 0.f, Rz0 = 0.f;
+                CT nz = CT(0);
+                if constexpr (!kWide) {
+                    nz = less(s_n[zn], nt.z);
+                    eval(s_st[zn], nz, Az, Rz);
+                    Az0 = s_A[zn];
+                    Rz0 = s_R[zn];
+                }
+                if constexpr (kPlus) {
+                    // the topic added to last: its A and R of one token more
+                    const int k = max(kp, 0);
+                    float A1, R1;
+                    eval(s_st[k], s_n[k] + 1, A1, R1);
+                    put_plus(kp >= 0, s_A + k, A1, R1);
+                }
                 const float r = __fmul_rn(u, total);
                 const bool in = nh > 0 && r < __fadd_rn(E, s);
                 int knew = 0;                        // the new topic (in the lane that keeps it)
@@ -366,58 +452,31 @@ k_infer_reg(InferArgs a)
                         if (r < __fadd_rn(E, w[t])) found = t;
                     found = in ? min(found, nh - 1) : max(nh - 1, 0);
                     knew = topic_of(found);
-                    // One lane forms the next token's removal (lane 31, which holds no
-                    // topic, with CH = 1, else the lane of that topic), every other lane
-                    // the addition to the topic it would draw.
-                    const bool mine = more_tokens && lane == (CH == 1 ? 31 : (zn >> 2) & 31);
-                    const int kx = mine ? zn : knew;
-                    const CT n = s_n[kx];
-                    CT nx = mine ? less(n, nt.z) : more(n, wt);
-                    // (the addition to the topic that the next token leaves)
-                    if (CH == 1 && more_tokens && !mine && knew == zn) nx = less(nx, nt.z);
+                    __syncwarp();                    // (the plus entries are renewed)
+                    // the topic this lane would draw with the token added -- and the next
+                    // one removed, if it leaves the same topic
+                    const bool same = more_tokens && knew == zn;
+                    CT nx = more(s_n[knew], wt);
                     float Ax, Rx;
-                    eval(s_st[kx], nx, Ax, Rx);
+                    if constexpr (kPlus) {
+                        Ax = s_Ap[knew];
+                        Rx = s_Rp[knew];
+                    } else {
+                        if (same) nx = less(nx, nt.z);
+                        eval(s_st[knew], nx, Ax, Rx);
+                    }
                     // the first lane that r falls in; topic K - 1 when rounding left it
                     // at or above the total
                     unsigned m = __ballot_sync(FULL, in);
                     if (m == 0) m = 1u << last_lane;
-                    const bool hit = (m & (0u - m)) == lt + 1u;
-                    keep = hit;
+                    keep = (m & (0u - m)) == lt + 1u;
                     __syncwarp();                    // every lane has read its entries
-                    if constexpr (CH == 1) {
-                        // the removal first: an addition to the same topic overwrites it
-                        if (mine) {
-                            s_n[kx] = nx;
-                            s_A[kx] = Ax;
-                            s_R[kx] = Rx;
-                        }
-                        __syncwarp();
-                        if (hit) {
-                            s_n[kx] = nx;
-                            s_A[kx] = Ax;
-                            s_R[kx] = Rx;
-                        }
-                    } else {
-                        if (hit && mine) {           // both in this lane
-                            CT n2 = more(s_n[knew], wt);
-                            if (knew == zn) n2 = less(n2, nt.z);
-                            float A2, R2;
-                            eval(s_st[knew], n2, A2, R2);
-                            if (knew == zn) {
-                                nx = n2;
-                                Ax = A2;
-                                Rx = R2;
-                            } else {
-                                s_n[knew] = n2;
-                                s_A[knew] = A2;
-                                s_R[knew] = R2;
-                            }
-                        }
-                        if (hit || mine) {
-                            s_n[kx] = nx;
-                            s_A[kx] = Ax;
-                            s_R[kx] = Rx;
-                        }
+                    // (integer counts: an addition and a removal of one topic leave it as it was)
+                    put(keep && !(kPlus && same), s_A + knew, nx, Ax, Rx);
+                    put(keep && more_tokens && !same, s_A + zn, nz, Az, Rz);
+                    if constexpr (kPlus) {
+                        put_plus(keep && more_tokens && !same, s_A + zn, Az0, Rz0);
+                        kp = keep && !same ? knew : -1;
                     }
                 } else {
                     const unsigned m = __ballot_sync(FULL, in);
@@ -439,7 +498,7 @@ k_infer_reg(InferArgs a)
                         float x2 = 0.f;
                         if (lane < nhh) x2 = __fmul_rn(s_A[at(k)], s_xs[lane]);
 #pragma unroll
-                        for (int i = 0; i < 5; ++i) x2 = hs_up(x2, 1 << i);
+                        for (int i = 0; i < 5; ++i) x2 = scan_step(x2, i);
                         const unsigned mb = __ballot_sync(FULL, lane < nhh && r < __fadd_rn(Eh, x2));
                         const int found = mb ? __ffs(mb) - 1 : nhh - 1;
                         knew = 128 * (found >> 2) + 4 * h + (found & 3);
@@ -454,26 +513,23 @@ k_infer_reg(InferArgs a)
                     eval(s_st[kx], nx, Ax, Rx);
                     keep = lane == 0;
                     __syncwarp();                    // every lane has read its entries
-                    if (lane == 0 || (lane == 1 && more_tokens && !both)) {
-                        s_n[at(kx)] = nx;
-                        s_A[at(kx)] = Ax;
-                        s_R[at(kx)] = Rx;
-                    }
+                    put(lane == 0 || (lane == 1 && more_tokens && !both), s_A + at(kx), nx, Ax, Rx);
                 }
-                if (keep) s_tok[jt & 63].x = __int_as_float(knew);
-                if (kind) {
-                    if (kind == 1) {
-                        if (keep) atomicAdd(&s_own[at(knew)], 1);
-                        if (lane == 0) atomicSub(&s_own[at(zn)], 1);
-                    } else {
-                        clear_own();
-                        if (kind == 3) start_run(jt + 1, nt);
-                    }
+                put_i(keep, &s_tok[jt & 63].x, knew);
+                add_own(keep && kind == 1, s_A + at(knew), 1);
+                add_own(lane == 0 && kind == 1, s_A + at(zn), -1);
+                if (kind >= 2) {
+                    if (in_run) clear_own();
+                    if (kind == 3) start_run(jt + 1, nt);
                 }
+                in_run = kind & 1;
                 __syncwarp();
                 tok = nt;
-#pragma unroll
-                for (int jj = 0; jj < CH; ++jj) g[jj] = gn[jj];
+              };
+#pragma unroll 1
+              for (uint32_t jt = base; jt < end; jt += 2) {      // (base is even)
+                  step(jt, ga, gb);
+                  if (jt + 1 < end) step(jt + 1, gb, ga);
               }
               if (base + lane < end) z[base + lane] = (uint16_t)__float_as_int(s_tok[(base + lane) & 63].x);
               __syncwarp();

@@ -167,7 +167,7 @@ struct Model {
     float* d_pcum = nullptr;
     float* d_ecum = nullptr;
     bool used = false;                  // a request was submitted: the model is frozen
-    bool nk_ok = true;                  // no negative n_k
+    uint64_t count_max = 0;             // no n_k or n_kw is larger (2^32 - 1: some may be negative)
     bool weighted = false;              // float counts (TermWeight IDF / PMI); requests carry weights
 };
 
@@ -395,7 +395,7 @@ bool server_step(tmt_server* s)
         a.esum = m->d_esum;
         a.pcum = m->d_pcum;
         a.ecum = m->d_ecum;
-        a.nk_ok = m->nk_ok;
+        a.small_counts = m->count_max + s->cfg.max_doc_len < (1u << 23);
         // every request of a model shares the draw key base; the per-request seed is folded in below
         a.key = 0;
         // requests may carry different seeds: launch per distinct seed (usually one)
@@ -580,9 +580,6 @@ tmt_status add_model_impl(tmt_server* s, uint32_t K, uint32_t V, const float* al
     m->asum_f = sf;
     m->asum_d = sd;
     m->weighted = weighted;
-    for (uint32_t k = 0; k < K && n_k; ++k)
-        if (!(weighted ? static_cast<const float*>(n_k)[k] >= 0.f : static_cast<const int32_t*>(n_k)[k] >= 0))
-            m->nk_ok = false;
     const uint32_t S = s->cfg.max_slots;
     m->slots = S;
     m->active.assign(S, -1);
@@ -635,6 +632,18 @@ tmt_status add_model_impl(tmt_server* s, uint32_t K, uint32_t V, const float* al
         if ((uint64_t)K * V)
             CK(cudaMemcpy(m->d_nkw, n_kw, (uint64_t)K * V * 4, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(m->d_nk, n_k, K * 4, cudaMemcpyHostToDevice));
+        if (weighted) {
+            for (uint32_t k = 0; k < K; ++k)
+                if (!(static_cast<const float*>(n_k)[k] >= 0.f)) m->count_max = 0xFFFFFFFFu;
+        } else {
+            uint32_t mx = 0;
+            CK(cudaMemset(m->d_counter, 0, sizeof(uint32_t)));
+            k_max_count<<<1184, 256>>>(m->d_nkw, (uint64_t)K * V, m->d_counter);
+            k_max_count<<<1, 256>>>(m->d_nk, K, m->d_counter);
+            CK(cudaGetLastError());
+            CK(cudaMemcpy(&mx, m->d_counter, sizeof(mx), cudaMemcpyDeviceToHost));
+            m->count_max = mx;
+        }
         CK(cudaMemcpy(m->d_alpha, alpha, K * sizeof(float), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(m->d_acum, acum.data(), K * sizeof(float), cudaMemcpyHostToDevice));
     } catch (const OomError&) {
