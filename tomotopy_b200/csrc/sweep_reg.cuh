@@ -25,11 +25,12 @@ constexpr uint64_t kRegMaxLen = 1ull << 24;
 constexpr int kRegWarps = 4;         // warps per block without split documents: one per SM sub-partition
 
 // resident blocks per SM (registers a thread may use): as many as leave the
-// token loop without spills worth the name
+// token loop without spills (6 blocks of 80 registers with CH = 1 spilled 40 bytes:
+// K = 100, 27.5M tokens, 10 sweeps 59-61 against 55 ms with 5)
 template <int CH, bool SPLIT, bool OPT>
 struct RegBlocks {
     static constexpr int value = SPLIT ? (CH <= 3 ? 2 : 1)
-                                       : CH <= 1 ? (OPT ? 5 : 6) : CH <= 2 ? (OPT ? 4 : 5) : CH <= 3 ? (OPT ? 3 : 4) : 3;
+                                       : CH <= 1 ? 5 : CH <= 2 ? 4 : 3;
 };
 
 //   CH: blocks of four topics per lane (K <= 128 CH)
@@ -73,6 +74,9 @@ k_sweep_reg(SweepArgs a)
     const int left = K - 4 * lane;
     const int nh = left <= 0 ? 0 : 4 * (left >> 7) + min(left & 127, 4);
     const unsigned last_bit = 1u << (((K - 1) >> 2) & 31);   // the lane of topic K - 1
+    float lm[5];                         // 1 in the lanes at or above 2^i, else 0
+#pragma unroll
+    for (int i = 0; i < 5; ++i) lm[i] = lane >= (1 << i) ? 1.f : 0.f;
     const float eta = a.eta, veta = a.veta;
     const uint32_t iter = a.iter_ptr ? *a.iter_ptr : a.iter;
 
@@ -165,8 +169,13 @@ k_sweep_reg(SweepArgs a)
         const float4* ph = phi4 + s_col[at & 63];
 #pragma unroll
         for (int jj = 0; jj < CH; ++jj)
-            p[jj] = 4 * lane + 128 * jj < KP ? __ldg(ph + 32 * jj) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (4 * lane + 128 * jj < KP) p[jj] = __ldg(ph + 32 * jj);
     };
+    // (a lane's blocks past K are never loaded and stay 0)
+#pragma unroll
+    for (int q = 0; q < kRing; ++q)
+#pragma unroll
+        for (int jj = 0; jj < CH; ++jj) pv[q][jj] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     // One draw: the token t4 = {topic, own weight, uniform, weight} at s_tok[j]
     // with column p; updates fn and leaves the new topic in s_tok[j].
@@ -195,9 +204,9 @@ k_sweep_reg(SweepArgs a)
         s = __fadd_rn(s, own_w);
         float x = s;
 #pragma unroll
-        for (int i = 0; i < STEPS; ++i) x = hs_up(x, 1 << i);
+        for (int i = 0; i < STEPS; ++i) x = hs_step(x, 1 << i, lm[i]);
         const float total = __shfl_sync(FULL, x, (1 << STEPS) - 1);
-        const float E = up1_or_0(x);
+        const float E = __fmul_rn(__shfl_up_sync(FULL, x, 1), lm[0]);
         // the prefix sums of this lane's own weights (Hillis-Steele order)
 #pragma unroll
         for (int off = 1; off < T; off <<= 1) {
@@ -222,7 +231,10 @@ k_sweep_reg(SweepArgs a)
 #pragma unroll
         for (int t = 0; t < T; ++t)
             if (sel == t) fn[t] = __fadd_rn(fn[t], WT ? wt : 1.f);
-        if (hit) s_tok[j].x = __int_as_float(topic_of(found));
+        // (predicated: a store under `if` is a branch on the draw's chain)
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p st.shared.s32 [%1], %2;\n}"
+                     :: "r"((int)hit), "r"((uint32_t)__cvta_generic_to_shared(s_tok + j)), "r"(topic_of(found))
+                     : "memory");
     };
 
     bool primed = false;                 // pv holds the first kRing - 1 columns of the coming draws
