@@ -211,13 +211,34 @@ __global__ void k_counts_rows(const uint64_t* __restrict__ doc_off, const uint32
 // ---------------------------------------------------------------------------
 // the training sweep
 // ---------------------------------------------------------------------------
-// Per-sweep word table: phi[v*KP + k] = ((float)n_kw[k,v] + eta) * R_k with
+// Per-group word table: phi[v*KP + k] = ((float)n_kw[k,v] + eta) * R_k with
 // R_k = 1 / ((float)n_k[k] + V*eta) and KP = K rounded up to a multiple of
-// 4 (entries K..KP-1 are 0); the same pass copies n_kw and n_k into the
-// next state, which the sweep then updates with the count deltas.
-__global__ void k_phi_copy(const int32_t* __restrict__ nkw, const int32_t* __restrict__ nk, uint32_t V, uint32_t K,
-                           uint32_t KP, float eta, float veta, float* __restrict__ phi, int32_t* __restrict__ nkw_next,
-                           int32_t* __restrict__ nk_next, uint32_t smem_k, PriorArgs pr, float* __restrict__ rm1)
+// 4 (entries K..KP-1 are 0 from the upload on); the same pass copies n_kw and n_k
+// into the next state, which the sweep then updates with the count deltas,
+// clears the sweep's document counters and, at the start of a captured sweep,
+// advances the sweep counter.
+// Bound by memory: 4 bytes read and 8 written per entry.  A block takes as many
+// words at a time as its threads cover with 16-byte accesses (K a multiple of 4
+// and no word priors), else all entries are dealt to the threads in their order in memory:
+// a block per word left most threads idle below K = 1024 and with element
+// accesses (V = 50,000, K = 100: 41 us; V = 10,000, K = 20: 11 us; V = 20,000,
+// K = 130: 20 us -- now 12, 5 and 14).
+constexpr uint32_t kPhiThreads = 256;
+
+// The counters the launch that follows needs (block 0).
+__device__ __forceinline__ void reset_counters(uint32_t* counter, uint32_t* step)
+{
+    if (blockIdx.x == 0) {
+        if (counter && threadIdx.x < 2) counter[threadIdx.x] = 0;
+        if (step && threadIdx.x == 0) *step += 1;
+    }
+}
+
+__global__ void __launch_bounds__(kPhiThreads)
+k_phi_copy(const int32_t* __restrict__ nkw, const int32_t* __restrict__ nk, uint32_t V, uint32_t K, uint32_t KP, float eta,
+           float veta, float* __restrict__ phi, int32_t* __restrict__ nkw_next, int32_t* __restrict__ nk_next,
+           uint32_t smem_k, PriorArgs pr, float* __restrict__ rm1, uint32_t* __restrict__ counter,
+           uint32_t* __restrict__ step)
 {
     extern __shared__ __align__(16) float s_R[];
     const bool r_smem = K <= smem_k;
@@ -229,16 +250,19 @@ __global__ void k_phi_copy(const int32_t* __restrict__ nkw, const int32_t* __res
             nk_next[k] = nk[k];
             rm1[k] = __fdiv_rn(1.0f, __fadd_rn((float)(nk[k] - 1), esum_of(pr, k, veta)));
         }
+    reset_counters(counter, step);
     __syncthreads();
     if (r_smem && (K & 3) == 0 && !pr.idx) {
-        // K a multiple of 4 (KP == K) and no word priors: 16-byte loads and
-        // stores, the same values
         const uint32_t K4 = K >> 2;
-        for (uint64_t v = blockIdx.x; v < V; v += gridDim.x) {
+        const uint32_t rows = max(1u, kPhiThreads / K4);         // words at a time
+        const uint32_t row = K4 < kPhiThreads ? threadIdx.x / K4 : 0;
+        if (row >= rows) return;
+        const uint32_t k0 = K4 < kPhiThreads ? threadIdx.x - row * K4 : threadIdx.x;
+        for (uint64_t v = (uint64_t)blockIdx.x * rows + row; v < V; v += (uint64_t)gridDim.x * rows) {
             const int4* src = reinterpret_cast<const int4*>(nkw + v * K);
             int4* dst = reinterpret_cast<int4*>(nkw_next + v * K);
             float4* ph = reinterpret_cast<float4*>(phi + v * KP);
-            for (uint32_t k4 = threadIdx.x; k4 < K4; k4 += blockDim.x) {
+            for (uint32_t k4 = k0; k4 < K4; k4 += kPhiThreads) {
                 const int4 n = __ldg(src + k4);
                 dst[k4] = n;
                 const float4 R = reinterpret_cast<const float4*>(s_R)[k4];
@@ -248,21 +272,21 @@ __global__ void k_phi_copy(const int32_t* __restrict__ nkw, const int32_t* __res
         }
         return;
     }
-    for (uint64_t v = blockIdx.x; v < V; v += gridDim.x) {
-        const int32_t* src = nkw + v * K;
-        int32_t* dst = nkw_next + v * K;
-        float* ph = phi + v * KP;
+    const uint64_t total = (uint64_t)V * K, stride = (uint64_t)gridDim.x * kPhiThreads;
+    const uint64_t dv = stride / K;
+    const uint32_t dk = (uint32_t)(stride - dv * K);
+    uint64_t i = (uint64_t)blockIdx.x * kPhiThreads + threadIdx.x;
+    uint64_t v = i / K;
+    uint32_t k = (uint32_t)(i - v * K);
+    for (; i < total; i += stride) {
+        const int32_t n = __ldg(nkw + i);
+        nkw_next[i] = n;
         const float* pe = prior_col(pr, v, K);
-        for (uint32_t k = threadIdx.x; k < KP; k += blockDim.x) {
-            float val = 0.f;
-            if (k < K) {
-                const int32_t n = src[k];
-                dst[k] = n;
-                const float R = r_smem ? s_R[k] : __fdiv_rn(1.0f, __fadd_rn((float)nk[k], esum_of(pr, k, veta)));
-                val = __fmul_rn(__fadd_rn((float)n, pe ? pe[k] : eta), R);
-            }
-            ph[k] = val;
-        }
+        const float R = r_smem ? s_R[k] : __fdiv_rn(1.0f, __fadd_rn((float)nk[k], esum_of(pr, k, veta)));
+        phi[v * KP + k] = __fmul_rn(__fadd_rn((float)n, pe ? pe[k] : eta), R);
+        v += dv;
+        k += dk;
+        if (k >= K) { k -= K; ++v; }
     }
 }
 
@@ -279,10 +303,12 @@ __global__ void k_nk_apply(int32_t* __restrict__ nk, int32_t* __restrict__ dnk, 
 
 __global__ void k_phi_apply(int32_t* __restrict__ nkw, int32_t* __restrict__ delta, const int32_t* __restrict__ nk,
                             uint32_t V, uint32_t K, uint32_t KP, float eta, float veta, float* __restrict__ phi,
-                            uint32_t smem_k, int fold, PriorArgs pr, float* __restrict__ rm1)
+                            uint32_t smem_k, int fold, PriorArgs pr, float* __restrict__ rm1,
+                            uint32_t* __restrict__ counter)
 {
     extern __shared__ float s_R[];
     const bool r_smem = phi && K <= smem_k;
+    reset_counters(counter, nullptr);
     if (r_smem)
         for (uint32_t k = threadIdx.x; k < K; k += blockDim.x)
             s_R[k] = __fdiv_rn(1.0f, __fadd_rn((float)nk[k], esum_of(pr, k, veta)));
@@ -358,10 +384,12 @@ __global__ void k_nk_fold_w(float* __restrict__ nk, long long* __restrict__ dk, 
 // n_kw fold (fold != 0) and, when phi != NULL, the word table of the state
 __global__ void k_phi_fold_w(float* __restrict__ nkw, long long* __restrict__ dkw, const float* __restrict__ nk,
                              uint32_t V, uint32_t K, uint32_t KP, float eta, float veta, float* __restrict__ phi,
-                             uint32_t smem_k, int fold, PriorArgs pr)
+                             uint32_t smem_k, int fold, PriorArgs pr, uint32_t* __restrict__ counter,
+                             uint32_t* __restrict__ step)
 {
     extern __shared__ float s_R[];
     const bool r_smem = phi && K <= smem_k;
+    reset_counters(counter, step);
     if (r_smem)
         for (uint32_t k = threadIdx.x; k < K; k += blockDim.x)
             s_R[k] = __fdiv_rn(1.0f, __fadd_rn(nk[k], esum_of(pr, k, veta)));
@@ -941,32 +969,89 @@ k_sweep_doc(SweepArgs a)
 // log-likelihood in FP64 (getLLDocs / getLLRest, LDAModel.hpp:616-668)
 // ---------------------------------------------------------------------------
 
+// The sum of n values in their order by one thread, the block staging them in
+// shared memory (kStage of them at a time); every thread calls it, thread 0 holds the sum.
+constexpr uint32_t kStage = 1024;
+
+template <typename S, typename F>
+__device__ S ordered_sum(uint32_t n, S* stage, F value)
+{
+    S s = S(0);
+    for (uint32_t b = 0; b < n; b += kStage) {
+        const uint32_t m = min(kStage, n - b);
+        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) stage[i] = value(b + i);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll 16
+            for (uint32_t i = 0; i < m; ++i) s = s + stage[i];
+        }
+        __syncthreads();
+    }
+    return s;
+}
+
 // n_dk rows and n_kw columns, each dealt to the warps in a fixed order, and
 // fixed reduction trees: bit-reproducible.
 // lg_alpha[k] = lgamma(alpha_k); asum[0] = sum(alpha), asum[1] = lgamma(sum(alpha))
 __global__ void k_ll_prep(const float* __restrict__ alpha, uint32_t K, double* __restrict__ lg_alpha,
                           double* __restrict__ asum)
 {
+    __shared__ double s_stage[kStage];
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) lg_alpha[k] = lgamma((double)alpha[k]);
+    const double s = ordered_sum<double>(K, s_stage, [&](uint32_t i) { return (double)alpha[i]; });
     if (threadIdx.x == 0) {
-        double s = 0;
-        for (uint32_t k = 0; k < K; ++k) s += (double)alpha[k];
         asum[0] = s;
         asum[1] = lgamma(s);
     }
 }
 
+// The terms of small integer counts, each the value k_ll_partials would form
+// itself: doc[n*K + k] = lgamma(n + alpha_k) - lg_alpha[k] (n < nd), word[n] =
+// lgamma(n + eta) - lg_eta (n < nw), len[n] = lgamma(n + sum(alpha)) -
+// lgamma(sum(alpha)) (n < nl).
+struct LlTab {
+    double* doc;
+    double* word;
+    double* len;
+    uint32_t nd, nw, nl;
+};
+
+__global__ void k_ll_tab(LlTab t, const float* __restrict__ alpha, uint32_t K, const double* __restrict__ lg_alpha,
+                         const double* __restrict__ asum_p, double eta, double lg_eta)
+{
+    const double asum = asum_p[0], lg_asum = asum_p[1];
+    const uint64_t nd = (uint64_t)t.nd * K, total = nd + t.nw + t.nl;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        if (i < nd) {
+            const uint32_t n = (uint32_t)(i / K), k = (uint32_t)(i - (uint64_t)n * K);
+            t.doc[i] = n ? lgamma((double)n + (double)alpha[k]) - lg_alpha[k] : 0.0;
+        } else if (i < nd + t.nw) {
+            const uint32_t n = (uint32_t)(i - nd);
+            t.word[n] = n ? lgamma((double)n + eta) - lg_eta : 0.0;
+        } else {
+            const uint32_t n = (uint32_t)(i - nd - t.nw);
+            t.len[n] = lgamma((double)n + asum) - lg_asum;
+        }
+    }
+}
+
 // CT: the count type (int32 for TermWeight ONE, float for weighted counts);
 // LT: the document length type (token count or weight sum).
-template <typename CT, typename LT>
+// TAB (integer counts): small counts' terms are read from k_ll_tab's tables.  An
+// FP64 lgamma takes a few hundred instructions and few of a row's counts are
+// nonzero, so evaluating them in place cost a warp nearly the whole row; with
+// the tables the counts' bytes bound the kernel.  The terms and their order are
+// the same, so the sums are the same bits.  K = 400, V = 30,000, 10M tokens (125 MB of counts): 200 -> 62 us.
+template <typename CT, typename LT, bool TAB>
 __global__ void k_ll_partials(const CT* __restrict__ ndk, uint64_t D, uint32_t K,
                               const double* __restrict__ lg_alpha, const float* __restrict__ alpha,
                               const LT* __restrict__ doc_len, const double* __restrict__ asum_p,
                               const CT* __restrict__ nkw, uint32_t V, double eta, double lg_eta,
                               double* __restrict__ partials, PriorArgs pr, const float* __restrict__ alpha_rows,
-                              const uint32_t* __restrict__ arow, const double* __restrict__ row_asum)
+                              const uint32_t* __restrict__ arow, const double* __restrict__ row_asum, LlTab tab)
 {
     __shared__ double s_d[32], s_r[32];
+    constexpr int kUnroll = 8;           // counts in flight per lane
     const double asum = asum_p[0], lg_asum = asum_p[1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -985,22 +1070,41 @@ __global__ void k_ll_partials(const CT* __restrict__ ndk, uint64_t D, uint32_t K
             if (lane == 0) accd -= lgamma((double)doc_len[r] + as_r) - lgas_r;
             continue;
         }
-        for (uint32_t k = lane; k < K; k += 32) {
-            const CT n = p[k];
-            if (n != CT(0)) accd += lgamma((double)n + (double)alpha[k]) - lg_alpha[k];
+        for (uint32_t k0 = lane; k0 < K; k0 += 32 * kUnroll) {
+            CT n[kUnroll];
+#pragma unroll
+            for (int i = 0; i < kUnroll; ++i) n[i] = k0 + 32 * i < K ? p[k0 + 32 * i] : CT(0);
+#pragma unroll
+            for (int i = 0; i < kUnroll; ++i) {
+                const uint32_t k = k0 + 32 * i;
+                if (n[i] != CT(0)) {
+                    if (TAB && (uint32_t)n[i] < tab.nd) accd += __ldg(tab.doc + (uint64_t)(uint32_t)n[i] * K + k);
+                    else accd += lgamma((double)n[i] + (double)alpha[k]) - lg_alpha[k];
+                }
+            }
         }
-        if (lane == 0) accd -= lgamma((double)doc_len[r] + asum) - lg_asum;
+        if (lane == 0) {
+            if (TAB && (uint32_t)doc_len[r] < tab.nl) accd -= __ldg(tab.len + (uint32_t)doc_len[r]);
+            else accd -= lgamma((double)doc_len[r] + asum) - lg_asum;
+        }
     }
     // the word rows' assignment does not depend on D: LLRest is the same bits on
     // every rank of a sharded corpus and on one GPU holding all of it
     for (uint64_t v = gw; v < V; v += nw) {
         const CT* p = nkw + v * K;
         const float* pe = prior_col(pr, v, K);
-        for (uint32_t k = lane; k < K; k += 32) {
-            const CT n = p[k];
-            if (n == CT(0)) continue;
-            if (pe) accr += lgamma((double)n + (double)pe[k]) - lgamma((double)pe[k]);
-            else accr += lgamma((double)n + eta) - lg_eta;
+        for (uint32_t k0 = lane; k0 < K; k0 += 32 * kUnroll) {
+            CT n[kUnroll];
+#pragma unroll
+            for (int i = 0; i < kUnroll; ++i) n[i] = k0 + 32 * i < K ? p[k0 + 32 * i] : CT(0);
+#pragma unroll
+            for (int i = 0; i < kUnroll; ++i) {
+                if (n[i] == CT(0)) continue;
+                const uint32_t k = k0 + 32 * i;
+                if (pe) accr += lgamma((double)n[i] + (double)pe[k]) - lgamma((double)pe[k]);
+                else if (TAB && (uint32_t)n[i] < tab.nw) accr += __ldg(tab.word + (uint32_t)n[i]);
+                else accr += lgamma((double)n[i] + eta) - lg_eta;
+            }
         }
     }
     accd = warp_sum(accd);
@@ -1096,27 +1200,79 @@ unsigned long long current_context_id()
 // ---------------------------------------------------------------------------
 // part_nom[bx*K + k] = sum over this block's docs of digammaApprox(n_dk + alpha_k)
 // part_den[bx]       = sum over this block's docs of digammaApprox(N_d + sum(alpha))
+// The sums keep the documents' order; what they add is formed apart from it.  A
+// digamma takes ~100 instructions and about a tenth of the counts of a row are
+// nonzero, so evaluating them where they stand ran at the cost of the whole row
+// (and, with K below a block's 256 threads, on K threads only).  Here all threads evaluate
+// a tile of documents x topics -- counts below 16 from the block's table of
+// digamma(n + alpha_k) -- and thread k then adds its column.  K = 1000, 120,000
+// documents: 462 -> 150 us; K = 100, 100,000 documents 129 -> 63 us; K = 20, 1,000
+// documents of 1,500 tokens 45 -> 9 us.
+constexpr uint32_t kAlphaThreads = 256;
+constexpr int kAlphaTab = 16;            // integer counts below this are looked up
+constexpr int kAlphaSteps = 8;           // counts a thread evaluates per tile
+
 template <typename CT, typename LT>
-__global__ void k_alpha_sums(const CT* __restrict__ ndk, uint64_t D, uint32_t K,
-                             const float* __restrict__ alpha, const LT* __restrict__ doc_len,
-                             const float* __restrict__ asum_p,
-                             double* __restrict__ part_nom, double* __restrict__ part_den)
+__global__ void __launch_bounds__(kAlphaThreads)
+k_alpha_sums(const CT* __restrict__ ndk, uint64_t D, uint32_t K, const float* __restrict__ alpha,
+             const LT* __restrict__ doc_len, const float* __restrict__ asum_p, double* __restrict__ part_nom,
+             double* __restrict__ part_den)
 {
+    constexpr bool kTab = std::is_same<CT, int32_t>::value;
     __shared__ double s_red[32];
+    __shared__ float s_val[kAlphaSteps * kAlphaThreads];
+    __shared__ float s_tab[kTab ? kAlphaTab * kAlphaThreads : 1];
+    __shared__ uint32_t s_nz[kAlphaThreads];
     const uint64_t per = (D + gridDim.x - 1) / gridDim.x;
-    const uint64_t d0 = blockIdx.x * per, d1 = min(D, d0 + per);
-    const uint32_t k = blockIdx.y * blockDim.x + threadIdx.x;
-    if (k < K) {
-        const float ak = alpha[k];
-        double acc = 0;
-        uint64_t zeros = 0;
-        for (uint64_t d = d0; d < d1; ++d) {
-            const CT n = ndk[d * K + k];
-            if (n != CT(0)) acc += (double)tmt::digamma_approx_f(__fadd_rn((float)n, ak));
-            else ++zeros;
+    const uint64_t d0 = min(D, blockIdx.x * per), d1 = min(D, d0 + per);
+    const uint32_t kb = blockIdx.y * kAlphaThreads;
+    const uint32_t cols = min(K - kb, kAlphaThreads), rows = kAlphaThreads / cols;   // a tile step's topics, documents
+    const uint32_t row = threadIdx.x / cols, col = threadIdx.x - row * cols;
+    const bool on = row < rows;
+    const float ak = alpha[kb + col];
+    if (row == 0) s_nz[col] = 0;
+    if constexpr (kTab) {
+        if (on)
+            for (uint32_t n = row; n < kAlphaTab; n += rows)
+                s_tab[n * cols + col] = n ? tmt::digamma_approx_f(__fadd_rn((float)n, ak)) : 0.f;
+    }
+    __syncthreads();
+    double acc = 0;
+    uint32_t nz = 0;
+    for (uint64_t d = d0; d < d1; d += (uint64_t)rows * kAlphaSteps) {
+        if (on) {
+            CT n[kAlphaSteps];
+#pragma unroll
+            for (int i = 0; i < kAlphaSteps; ++i) {
+                const uint64_t dd = d + (uint64_t)i * rows + row;
+                n[i] = dd < d1 ? ndk[dd * K + kb + col] : CT(0);
+            }
+#pragma unroll
+            for (int i = 0; i < kAlphaSteps; ++i) {
+                float v = 0.f;
+                if (n[i] != CT(0)) {
+                    ++nz;
+                    if (kTab && n[i] > CT(0) && n[i] < CT(kAlphaTab)) v = s_tab[(uint32_t)n[i] * cols + col];
+                    else v = tmt::digamma_approx_f(__fadd_rn((float)n[i], ak));
+                }
+                s_val[(i * rows + row) * cols + col] = v;
+            }
         }
+        __syncthreads();
+        if (row == 0) {
+            // (a zero count adds 0 here and counts below)
+            const uint32_t m = (uint32_t)min((uint64_t)rows * kAlphaSteps, d1 - d);
+#pragma unroll 8
+            for (uint32_t i = 0; i < m; ++i) acc += (double)s_val[i * cols + col];
+        }
+        __syncthreads();
+    }
+    if (on && nz) atomicAdd(&s_nz[col], nz);
+    __syncthreads();
+    if (row == 0) {
+        const uint64_t zeros = (d1 - d0) - s_nz[col];
         acc += (double)zeros * (double)tmt::digamma_approx_f(ak);
-        part_nom[(uint64_t)blockIdx.x * K + k] = acc;
+        part_nom[(uint64_t)blockIdx.x * K + kb + col] = acc;
     }
     if (blockIdx.y == 0) {
         const float as = *asum_p;
@@ -1135,33 +1291,63 @@ __global__ void k_alpha_sums(const CT* __restrict__ ndk, uint64_t D, uint32_t K,
     }
 }
 
-// One fixed-point step for every k, then the new sum(alpha) for the next step.
-__global__ void k_alpha_update(const double* __restrict__ part_nom, const double* __restrict__ part_den,
-                               uint32_t nparts, uint32_t K, uint64_t D, float* __restrict__ alpha,
-                               float* __restrict__ asum_p, const float* __restrict__ dg_points)
+// One fixed-point step: block b takes topics [64 b, 64 b + 64), each of its first
+// 64 threads adding its topic's partial sums in order (16 loads in flight), a third
+// warp meanwhile the length sums; the last block to finish forms the new
+// sum(alpha), in order.  Bound by the chain of dependent FP64 adds.  (One block for all
+// topics, its serial sums read from global memory: 118 us at 592 partial sums; now 32.)
+constexpr uint32_t kAlphaUpd = 64;
+
+__global__ void __launch_bounds__(kAlphaUpd + 32)
+k_alpha_update(const double* __restrict__ part_nom, const double* __restrict__ part_den, uint32_t nparts, uint32_t K,
+               uint64_t D, float* __restrict__ alpha, float* __restrict__ asum_p, const float* __restrict__ dg_points,
+               uint32_t* __restrict__ done)
 {
+    __shared__ double s_stage[kStage];
     __shared__ double s_den;
+    __shared__ bool s_last;
     tmt::DigammaTable dg{ dg_points };
-    if (threadIdx.x == 0) {
-        double den = 0;
-        for (uint32_t i = 0; i < nparts; ++i) den += part_den[i];
-        s_den = den - (double)D * (double)dg(*asum_p);
+    // (nparts <= kStage: n_apart)
+    for (uint32_t i = threadIdx.x; i < nparts; i += blockDim.x) s_stage[i] = part_den[i];
+    __syncthreads();
+    if (threadIdx.x == kAlphaUpd) {
+        double sum = 0;
+#pragma unroll 16
+        for (uint32_t i = 0; i < nparts; ++i) sum += s_stage[i];
+        s_den = sum - (double)D * (double)dg(*asum_p);
+    }
+    const uint32_t k = blockIdx.x * kAlphaUpd + threadIdx.x;
+    const bool on = threadIdx.x < kAlphaUpd && k < K;
+    double nom = 0;
+    float ak = 0.f;
+    if (on) {
+        uint32_t i = 0;
+        for (; i + 16 <= nparts; i += 16) {
+            double x[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = __ldg(part_nom + (uint64_t)(i + j) * K + k);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) nom += x[j];
+        }
+        for (; i < nparts; ++i) nom += part_nom[(uint64_t)i * K + k];
+        ak = alpha[k];
+        nom -= (double)D * (double)dg(ak);
     }
     __syncthreads();
-    const double den = s_den;
-    for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) {
-        double nom = 0;
-        for (uint32_t i = 0; i < nparts; ++i) nom += part_nom[(uint64_t)i * K + k];
-        const float ak = alpha[k];
-        nom -= (double)D * (double)dg(ak);
-        const float na = __fmul_rn(__fdiv_rn((float)nom, (float)den), ak);
+    if (on) {
+        const float na = __fmul_rn(__fdiv_rn((float)nom, (float)s_den), ak);
         alpha[k] = na > 1e-5f ? na : 1e-5f;
     }
+    __threadfence();
     __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const float s = ordered_sum<float>(K, reinterpret_cast<float*>(s_stage), [&](uint32_t i) { return __ldcg(alpha + i); });
     if (threadIdx.x == 0) {
-        float s = 0.f;
-        for (uint32_t k = 0; k < K; ++k) s = __fadd_rn(s, alpha[k]);
         *asum_p = s;
+        *done = 0;
     }
 }
 
@@ -1181,24 +1367,21 @@ __global__ void k_alpha_fold(const double* __restrict__ part_nom, const double* 
     }
 }
 
-// the sweep counter of captured sweeps: set before a run of graph launches,
-// advanced by the last node of each
+// the sweep counter of captured sweeps: set to the sweep before the first one of a
+// run of graph launches, advanced by the first node of each
 __global__ void k_set_step(uint32_t* __restrict__ step, uint32_t v)
 {
     *step = v;
 }
 
-__global__ void k_next_step(uint32_t* __restrict__ step)
+__global__ void k_sum_alpha(const float* __restrict__ alpha, uint32_t K, float* __restrict__ out,
+                            uint32_t* __restrict__ done)
 {
-    *step += 1;
-}
-
-__global__ void k_sum_alpha(const float* __restrict__ alpha, uint32_t K, float* __restrict__ out)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        float s = 0.f;
-        for (uint32_t k = 0; k < K; ++k) s = __fadd_rn(s, alpha[k]);
+    __shared__ float s_stage[kStage];
+    const float s = ordered_sum<float>(K, s_stage, [&](uint32_t i) { return alpha[i]; });
+    if (threadIdx.x == 0) {
         *out = s;
+        *done = 0;
     }
 }
 
@@ -1461,7 +1644,7 @@ void host_copy_parallel(char* dst, const char* src, uint64_t bytes, uint32_t max
     for (auto& x : th) x.join();
 }
 
-constexpr uint64_t kStageChunk = 32ull << 20;   // a staging buffer; staged transfers are >= 32 MB
+constexpr uint64_t kStageChunk = 32ull << 20;   // a staging buffer
 
 // true for memory CUDA knows (pinned host, device or managed memory): one
 // direct copy serves it; false for plain pageable host memory
@@ -1842,10 +2025,9 @@ void do_sweep_sharded(tmt_handle* h)
         }
         k_phi_apply<<<grid, 256, smem_k * 4, h->stream>>>(h->d_nkw[0], dnkw, h->d_nk[0], V, K, round4(K), h->cfg.eta,
                                                         veta, h->d_phi, smem_k, pending ? 1 : 0, h->prior_args(),
-                                                        h->d_rm1);
+                                                        h->d_rm1, h->d_counter);
         launch_check(h);
         if (h->group_bounds[g] < h->group_bounds[g + 1]) {
-            CK(cudaMemsetAsync(h->d_counter, 0, 2 * sizeof(uint32_t), h->stream));
             tune_mark(h, g, 0);
             launch_sweep(h, sweep_args(h, h->d_nkw[0], h->d_nk[0], dnkw, dnk, g), variant_of(h, g));
             tune_mark(h, g, 1);
@@ -1857,7 +2039,7 @@ void do_sweep_sharded(tmt_handle* h)
         k_nk_apply<<<1, 1024, 0, h->stream>>>(h->d_nk[0], dnk, K);
         launch_check(h);
         k_phi_apply<<<grid, 256, 0, h->stream>>>(h->d_nkw[0], dnkw, h->d_nk[0], V, K, round4(K), h->cfg.eta, veta,
-                                                nullptr, 0, 1, h->prior_args(), nullptr);
+                                                nullptr, 0, 1, h->prior_args(), nullptr, nullptr);
         launch_check(h);
     }
     CK(cudaEventRecord(h->kev1, h->stream));
@@ -1895,9 +2077,9 @@ void do_sweep_w(tmt_handle* h, bool capture)
         if (h->group_bounds[g] == h->group_bounds[g + 1]) continue;
         if (pending) fold_nk();
         k_phi_fold_w<<<grid, 256, smem_k * 4, h->stream>>>(nkw, h->d_dkw, nk, V, K, round4(K), h->cfg.eta, veta,
-                                                         h->d_phi, smem_k, pending ? 1 : 0, h->prior_args());
+                                                         h->d_phi, smem_k, pending ? 1 : 0, h->prior_args(),
+                                                         h->d_counter, capture && !pending ? h->d_step : nullptr);
         launch_check(h);
-        CK(cudaMemsetAsync(h->d_counter, 0, 2 * sizeof(uint32_t), h->stream));
         SweepArgs a = sweep_args(h, h->d_nkw[0], h->d_nk[0], nullptr, nullptr, g);
         a.wt = h->d_wt;
         a.dkw = h->d_dkw;
@@ -1914,7 +2096,7 @@ void do_sweep_w(tmt_handle* h, bool capture)
     if (pending) {
         fold_nk();
         k_phi_fold_w<<<grid, 256, 0, h->stream>>>(nkw, h->d_dkw, nk, V, K, round4(K), h->cfg.eta, veta, nullptr, 0, 1,
-                                                 h->prior_args());
+                                                 h->prior_args(), nullptr, nullptr);
         launch_check(h);
     }
     if (!capture) {
@@ -1935,18 +2117,20 @@ void do_sweep(tmt_handle* h, bool capture = false)
     if (h->weighted) return do_sweep_w(h, capture);
     const uint32_t K = h->cfg.K, V = h->cfg.V;
     const float veta = h->cfg.eta * (float)V;
-    bool recorded = false;
+    bool recorded = false, first = true;
     const uint32_t G = (uint32_t)h->group_bounds.size() - 1;
     for (uint32_t g = 0; g < G; ++g) {
         if (h->group_bounds[g] == h->group_bounds[g + 1]) continue;
         const int cur = h->cur, nxt = cur ^ 1;
         const uint32_t smem_k = K <= 12288 ? K : 0;
-        uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)h->num_sms * 16, V));
-        k_phi_copy<<<grid, 256, smem_k * 4, h->stream>>>(h->d_nkw[cur], h->d_nk[cur], V, K, round4(K), h->cfg.eta,
-                                                        veta, h->d_phi, h->d_nkw[nxt], h->d_nk[nxt], smem_k,
-                                                        h->prior_args(), h->d_rm1);
+        // about 8 entries a thread and pass, at most 16 blocks an SM
+        const uint32_t grid = (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>((uint64_t)h->num_sms * 16, ((uint64_t)V * K + 8 * kPhiThreads - 1) / (8 * kPhiThreads)));
+        k_phi_copy<<<grid, kPhiThreads, smem_k * 4, h->stream>>>(
+            h->d_nkw[cur], h->d_nk[cur], V, K, round4(K), h->cfg.eta, veta, h->d_phi, h->d_nkw[nxt], h->d_nk[nxt], smem_k,
+            h->prior_args(), h->d_rm1, h->d_counter, capture && first ? h->d_step : nullptr);
         launch_check(h);
-        CK(cudaMemsetAsync(h->d_counter, 0, 2 * sizeof(uint32_t), h->stream));
+        first = false;
         SweepArgs a = sweep_args(h, h->d_nkw[cur], h->d_nk[cur], h->d_nkw[nxt], h->d_nk[nxt], g);
         if (capture) a.iter_ptr = h->d_step;
         if (!capture) {
@@ -1966,7 +2150,7 @@ void do_sweep(tmt_handle* h, bool capture = false)
 
 // One sweep as a graph launch: the sweep's launches are captured once per
 // starting buffer parity (after the autotuner has fixed every group's
-// variant) and replayed; the last node advances the device sweep counter.
+// variant) and replayed; the first node advances the device sweep counter.
 void graph_sweep(tmt_handle* h)
 {
     const int p = h->cur;
@@ -1977,8 +2161,6 @@ void graph_sweep(tmt_handle* h)
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         try {
             do_sweep(h, true);
-            k_next_step<<<1, 1, 0, h->stream>>>(h->d_step);
-            launch_check(h);
         } catch (...) {
             cudaStreamEndCapture(h->stream, &g);
             if (g) cudaGraphDestroy(g);
@@ -2008,16 +2190,17 @@ void graph_sweep(tmt_handle* h)
 void do_optimize(tmt_handle* h)
 {
     const uint32_t K = h->cfg.K;
-    dim3 grid(h->n_apart, (K + 255) / 256);
-    k_sum_alpha<<<1, 32, 0, h->stream>>>(h->d_alpha, K, h->d_asum);
+    dim3 grid(h->n_apart, (K + kAlphaThreads - 1) / kAlphaThreads);
+    // (the sweep is over: its document counter serves k_alpha_update)
+    k_sum_alpha<<<1, 256, 0, h->stream>>>(h->d_alpha, K, h->d_asum, h->d_counter);
     launch_check(h);
     for (int it = 0; it < 10; ++it) {
         if (h->weighted)
-            k_alpha_sums<<<grid, 256, 0, h->stream>>>(reinterpret_cast<const float*>(h->d_ndk), h->D, K, h->d_alpha,
+            k_alpha_sums<<<grid, kAlphaThreads, 0, h->stream>>>(reinterpret_cast<const float*>(h->d_ndk), h->D, K, h->d_alpha,
                                                       (const float*)h->d_doc_wlen, h->d_asum, h->d_part_nom,
                                                       h->d_part_den);
         else
-            k_alpha_sums<<<grid, 256, 0, h->stream>>>(h->d_ndk, h->n_rows ? h->n_rows : h->D, K, h->d_alpha,
+            k_alpha_sums<<<grid, kAlphaThreads, 0, h->stream>>>(h->d_ndk, h->n_rows ? h->n_rows : h->D, K, h->d_alpha,
                                                       h->d_doc_len, h->d_asum, h->d_part_nom, h->d_part_den);
         launch_check(h);
         uint32_t nparts = h->n_apart;
@@ -2033,8 +2216,8 @@ void do_optimize(tmt_handle* h)
             nom = h->d_alpha_fold;
             den = h->d_alpha_fold + K;
         }
-        k_alpha_update<<<1, 1024, 0, h->stream>>>(nom, den, nparts, K, h->n_rows ? h->n_rows : h->D_global,
-                                                  h->d_alpha, h->d_asum, h->d_dg_points);
+        k_alpha_update<<<(K + kAlphaUpd - 1) / kAlphaUpd, kAlphaUpd + 32, 0, h->stream>>>(
+            nom, den, nparts, K, h->n_rows ? h->n_rows : h->D_global, h->d_alpha, h->d_asum, h->d_dg_points, h->d_counter);
         launch_check(h);
     }
 }
@@ -2049,20 +2232,40 @@ void do_ll(tmt_handle* h, double* d_out)
     k_ll_prep<<<1, 256, 0, h->stream>>>(h->d_alpha, K, h->d_lg_alpha, h->d_asum_ll);
     launch_check(h);
     if (h->weighted) {
-        k_ll_partials<<<h->n_partials, 256, 0, h->stream>>>(
+        k_ll_partials<float, float, false><<<h->n_partials, 256, 0, h->stream>>>(
             reinterpret_cast<const float*>(h->d_ndk), h->D, K, h->d_lg_alpha, h->d_alpha, (const float*)h->d_doc_wlen,
             h->d_asum_ll, reinterpret_cast<const float*>(h->d_nkw[0]), h->cfg.V, eta, std::lgamma(eta), h->d_partials,
-            h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum);
+            h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum, LlTab{});
         launch_check(h);
         k_ll_final<<<1, 256, 0, h->stream>>>(h->d_partials, h->n_partials, reinterpret_cast<const float*>(h->d_nk[0]),
                                              K, veta, d_out, h->d_esum);
     } else {
-        k_ll_partials<<<h->n_partials, 256, 0, h->stream>>>(h->d_ndk, h->n_rows ? h->n_rows : h->D, K,
-                                                            h->d_lg_alpha, h->d_alpha,
-                                                            h->d_doc_len, h->d_asum_ll,
-                                                            h->d_nkw[h->cur], h->cfg.V, eta, std::lgamma(eta),
-                                                            h->d_partials, h->prior_args(), h->d_alpha_rows,
-                                                            h->d_arow, h->d_row_asum);
+        // the tables lie in the alpha optimiser's partial sums, which are free here: as
+        // many document rows as an eighth of them hold, the rest to the others
+        const uint64_t rows = h->n_rows ? h->n_rows : h->D, room = (uint64_t)h->n_apart * K;
+        LlTab t{};
+        t.nd = (uint32_t)std::min<uint64_t>(1024, h->n_apart / 2);
+        t.nw = (uint32_t)std::min<uint64_t>(4096, room / 4);
+        t.nl = (uint32_t)std::min<uint64_t>(4096, room / 4);
+        t.doc = h->d_part_nom;
+        t.word = t.doc + (uint64_t)t.nd * K;
+        t.len = t.word + t.nw;
+        // (not for states whose counts are fewer than the tables' entries)
+        const uint64_t entries = (uint64_t)t.nd * K + t.nw + t.nl;
+        const bool use_tab = rows * K + (uint64_t)K * h->cfg.V >= 4 * entries;
+        const double lg_eta = std::lgamma(eta);
+        if (use_tab) {
+            k_ll_tab<<<(uint32_t)std::min<uint64_t>((entries + 255) / 256, (uint64_t)h->num_sms * 8), 256, 0, h->stream>>>(
+                t, h->d_alpha, K, h->d_lg_alpha, h->d_asum_ll, eta, lg_eta);
+            launch_check(h);
+            k_ll_partials<int32_t, int32_t, true><<<h->n_partials, 256, 0, h->stream>>>(
+                h->d_ndk, rows, K, h->d_lg_alpha, h->d_alpha, h->d_doc_len, h->d_asum_ll, h->d_nkw[h->cur], h->cfg.V, eta,
+                lg_eta, h->d_partials, h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum, t);
+        } else {
+            k_ll_partials<int32_t, int32_t, false><<<h->n_partials, 256, 0, h->stream>>>(
+                h->d_ndk, rows, K, h->d_lg_alpha, h->d_alpha, h->d_doc_len, h->d_asum_ll, h->d_nkw[h->cur], h->cfg.V, eta,
+                lg_eta, h->d_partials, h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum, t);
+        }
         launch_check(h);
         k_ll_final<<<1, 256, 0, h->stream>>>(h->d_partials, h->n_partials, h->d_nk[h->cur], K, veta, d_out,
                                              h->d_esum);
@@ -2353,7 +2556,8 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
         h->d_ll = nullptr;
         const std::vector<float>& dg = tmt::digamma_points();
         h->d_dg_points = h->dalloc<float>(dg.size());
-        h->n_apart = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)h->num_sms * 4, (D + 63) / 64));
+        h->n_apart = (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>({ (uint64_t)h->num_sms * 4, (D + 63) / 64, kStage }));
         h->d_part_nom = h->dalloc<double>((size_t)h->n_apart * K);
         h->d_part_den = h->dalloc<double>(h->n_apart);
 
@@ -2366,6 +2570,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
         CK(cudaMemsetAsync(h->d_ndk, 0, D * (uint64_t)K * sizeof(int32_t), st));
         CK(cudaMemsetAsync(h->d_nkw[0], 0, (uint64_t)K * V * sizeof(int32_t), st));
         CK(cudaMemsetAsync(h->d_nk[0], 0, K * sizeof(int32_t), st));
+        if (K & 3) CK(cudaMemsetAsync(h->d_phi, 0, (uint64_t)round4(K) * V * sizeof(float), st));   // its padding
         if (z0) {
             h2d(h, h->d_z, z0, n_all * sizeof(uint16_t));
         } else if (n_all) {
@@ -2394,7 +2599,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
             const uint32_t g2 = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)h->num_sms * 16, V));
             k_phi_fold_w<<<g2, 256, 0, st>>>(reinterpret_cast<float*>(h->d_nkw[0]), h->d_dkw,
                                              reinterpret_cast<const float*>(h->d_nk[0]), V, K, round4(K), h->cfg.eta,
-                                             h->cfg.eta * (float)V, nullptr, 0, 1, h->prior_args());
+                                             h->cfg.eta * (float)V, nullptr, 0, 1, h->prior_args(), nullptr, nullptr);
             launch_check(h);
             // the token counts per document as well (the shard planner's facts)
             CK(cudaMemcpyAsync(h->d_doc_len, len.data(), D * sizeof(int32_t), cudaMemcpyHostToDevice, st));
@@ -2555,7 +2760,7 @@ tmt_status tmt_train(tmt_handle* h, uint32_t iters, uint32_t ll_every, double* l
         for (uint32_t i = 0; i < iters; ++i) {
             if (use_graphs && h->tuned >= 0) {
                 if (!in_run) {
-                    k_set_step<<<1, 1, 0, h->stream>>>(h->d_step, (uint32_t)h->global_step);
+                    k_set_step<<<1, 1, 0, h->stream>>>(h->d_step, (uint32_t)h->global_step - 1u);
                     launch_check(h);
                     CK(cudaEventRecord(run_event(2 * runs), h->stream));
                     in_run = true;
@@ -3248,8 +3453,9 @@ tmt_status tmt_ll_counts_noalloc(const int32_t* n_dk, uint64_t D, uint32_t K, co
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const double etad = (double)eta;
     k_ll_prep<<<1, 256, 0, st>>>(alpha, K, lg_alpha, asum);
-    k_ll_partials<<<blocks, 256, 0, st>>>(n_dk, D, K, lg_alpha, alpha, doc_len, asum, n_kw, V, etad,
-                                          std::lgamma(etad), partials, PriorArgs{}, nullptr, nullptr, nullptr);
+    k_ll_partials<int32_t, int32_t, false><<<blocks, 256, 0, st>>>(n_dk, D, K, lg_alpha, alpha, doc_len, asum, n_kw, V,
+                                                                   etad, std::lgamma(etad), partials, PriorArgs{},
+                                                                   nullptr, nullptr, nullptr, LlTab{});
     k_ll_final<<<1, 256, 0, st>>>(partials, blocks, n_k, K, (double)V * etad, ll_out, nullptr);
     // no error was pending before the launches: one now is theirs
     e = cudaGetLastError();
