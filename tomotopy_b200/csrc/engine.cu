@@ -964,6 +964,7 @@ k_sweep_doc(SweepArgs a)
 }
 
 #include "sweep_reg.cuh"
+#include "sweep_wide.cuh"
 
 // ---------------------------------------------------------------------------
 // log-likelihood in FP64 (getLLDocs / getLLRest, LDAModel.hpp:616-668)
@@ -1825,10 +1826,10 @@ void launch_sweep_t(tmt_handle* h, const SweepArgs& a, const SweepShape& sh)
 // two of the tuner's sweeps spent on it; at K = 1000, the word's column
 // read from L1 every token, 6 blocks/SM, and a per-warp shared-memory copy
 // of it -- fewer instructions, slower sweeps.)
-// K <= kRegMaxK (k_sweep_reg) and K > 4096 have one variant.
+// K <= kWideMaxK (k_sweep_reg, k_sweep_wide) and K > 4096 have one variant.
 int sweep_variants_for(uint32_t K)
 {
-    return K <= kRegMaxK || (round4(K) + 127) / 128 > 32 ? 1 : 2;
+    return K <= kWideMaxK || (round4(K) + 127) / 128 > 32 ? 1 : 2;
 }
 
 template <int CH, bool WT, bool PLAIN>
@@ -1861,7 +1862,6 @@ void launch_sweep_w(tmt_handle* h, const SweepArgs& b, const SweepShape& sh, uin
         if (b.n_long) return launch_sweep_t<0, 3, false, true>(h, b, sh);
     }
     if (ch <= 4) launch_sweep_t<0, 3, WT>(h, b, sh);     // as above, not split
-    else if (ch <= 8) launch_sweep_ch<8, WT>(h, b, sh, variant, plain);
     else if (ch <= 16) launch_sweep_ch<16, WT>(h, b, sh, variant, plain);
     else if (ch <= 32) launch_sweep_ch<32, WT>(h, b, sh, variant, plain);
     else launch_sweep_t<0, 3, WT>(h, b, sh);
@@ -1909,8 +1909,51 @@ void launch_reg(tmt_handle* h, const SweepArgs& a)
     else launch_reg_ch<4, 5>(h, a);
 }
 
+// --- k_sweep_wide: 256 < K <= kWideMaxK ---
+template <int CH, typename NT, bool OPT>
+void launch_wide_t(tmt_handle* h, const SweepArgs& a)
+{
+    auto kern = k_sweep_wide<CH, NT, OPT>;
+    const uint32_t smem = 128 * CH * (8 + kWideWarps * (4 + (uint32_t)sizeof(NT)));
+    int per_sm = 0;
+    for (const auto& e : h->occ)
+        if (e.kern == (const void*)kern) per_sm = e.per_sm;
+    if (per_sm == 0) {
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWideWarps * 32, smem));
+        if (per_sm < 1) throw CudaError("sweep kernel does not fit on an SM");
+        h->occ.push_back({ (const void*)kern, smem, per_sm });
+    }
+    const uint32_t grid = (uint32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>((uint64_t)per_sm * h->num_sms, (a.pos_end - a.pos_begin + kWideWarps - 1) / kWideWarps));
+    kern<<<grid, kWideWarps * 32, smem, h->stream>>>(a);
+    launch_check(h);
+}
+
+template <int CH>
+void launch_wide_ch(tmt_handle* h, const SweepArgs& a)
+{
+    const bool opt = a.arow || a.mask;
+    if (a.wt) opt ? launch_wide_t<CH, float, true>(h, a) : launch_wide_t<CH, float, false>(h, a);
+    else if (a.max_len >= 65536) launch_wide_t<CH, int, true>(h, a);
+    else opt ? launch_wide_t<CH, uint16_t, true>(h, a) : launch_wide_t<CH, uint16_t, false>(h, a);
+}
+
 void launch_sweep(tmt_handle* h, const SweepArgs& a, int variant)
 {
+    // k_sweep_wide above kRegMaxK, and from 257 topics on where the launch has documents
+    // enough (16 an SM) that instructions bound it, not the chain of the longest: K = 333,
+    // 4.9M tokens, 10 sweeps 28.1 -> 26.9 ms (at K = 130, 17.9 -> 19.7: not below 257)
+    if (a.K <= kWideMaxK &&
+        (a.K > kRegMaxK || (a.K > 256 && !a.n_long && a.pos_end - a.pos_begin >= (uint64_t)h->num_sms * 16))) {
+        if (a.K <= 384) launch_wide_ch<3>(h, a);
+        else if (a.K <= 512) launch_wide_ch<4>(h, a);
+        else if (a.K <= 640) launch_wide_ch<5>(h, a);
+        else if (a.K <= 768) launch_wide_ch<6>(h, a);
+        else if (a.K <= 896) launch_wide_ch<7>(h, a);
+        else launch_wide_ch<8>(h, a);
+        return;
+    }
     if (a.K <= kRegMaxK && a.max_len < kRegMaxLen) return launch_reg(h, a);
     const uint32_t KP = round4(a.K);
     const uint32_t ch = (KP + 127) / 128;
