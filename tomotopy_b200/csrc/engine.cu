@@ -1894,7 +1894,7 @@ template <int CH, int STEPS>
 void launch_reg_ch(tmt_handle* h, const SweepArgs& a)
 {
     const bool opt = a.arow || a.mask;
-    if (a.wt) launch_reg_t<CH, STEPS, true, false, true>(h, a);
+    if (a.wt) opt ? launch_reg_t<CH, STEPS, true, false, true>(h, a) : launch_reg_t<CH, STEPS, true, false, false>(h, a);
     else if (a.n_long) opt ? launch_reg_t<CH, STEPS, false, true, true>(h, a) : launch_reg_t<CH, STEPS, false, true, false>(h, a);
     else opt ? launch_reg_t<CH, STEPS, false, false, true>(h, a) : launch_reg_t<CH, STEPS, false, false, false>(h, a);
 }

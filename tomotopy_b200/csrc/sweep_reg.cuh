@@ -26,10 +26,11 @@ constexpr int kRegWarps = 4;         // warps per block without split documents:
 
 // resident blocks per SM (registers a thread may use): as many as leave the
 // token loop without spills (6 blocks of 80 registers with CH = 1 spilled 40 bytes:
-// K = 100, 27.5M tokens, 10 sweeps 59-61 against 55 ms with 5)
+// K = 100, 27.5M tokens, 10 sweeps 59-61 against 55 ms with 5; split documents at
+// 2 blocks of 8 warps spilled 40-140 with CH = 2 and 3: K = 333 26.9 against 25.4 ms)
 template <int CH, bool SPLIT, bool OPT>
 struct RegBlocks {
-    static constexpr int value = SPLIT ? (CH <= 3 ? 2 : 1)
+    static constexpr int value = SPLIT ? (CH <= 1 ? 2 : 1)
                                        : CH <= 1 ? 5 : CH <= 2 ? 4 : 3;
 };
 
@@ -62,7 +63,7 @@ k_sweep_reg(SweepArgs a)
     uint32_t* s_col = s_col_all[warp];
     for (int i = lane; i < 64; i += 32) s_col[i] = 0;    // (read ahead of what is written: any column)
     __syncwarp();
-    int* s_dnk = smem;                   // n_k deltas of the block (integer counts)
+    int* s_dnk = smem;                   // n_k deltas of the block (integer counts): its rows' changes
     int* s_dlt = smem + KP;              // SPLIT: three step buffers of the document's row changes
     __shared__ uint32_t s_q;
     if (!WT) {
@@ -165,8 +166,8 @@ k_sweep_reg(SweepArgs a)
 
     float4 pv[kRing][CH];                // columns of the word table: token j in pv[j % kRing]
     const float4* phi4 = reinterpret_cast<const float4*>(a.phi) + lane;
-    auto load_col = [&](uint32_t at, float4 (&p)[CH]) {
-        const float4* ph = phi4 + s_col[at & 63];
+    auto load_col = [&](uint32_t col, float4 (&p)[CH]) {
+        const float4* ph = phi4 + col;
 #pragma unroll
         for (int jj = 0; jj < CH; ++jj)
             if (4 * lane + 128 * jj < KP) p[jj] = __ldg(ph + 32 * jj);
@@ -197,6 +198,7 @@ k_sweep_reg(SweepArgs a)
             const float4 q = p[t >> 2];
             const float pt = (t & 3) == 0 ? q.x : (t & 3) == 1 ? q.y : (t & 3) == 2 ? q.z : q.w;
             // the own topic is left out of the chain (its product is 0) and added last
+            // (products with a 0/1 vector in place of the selects measured slower)
             s = __fmaf_rn(A[t], own ? 0.f : pt, s);
             w[t] = __fmul_rn(A[t], own ? po : pt);
             if (own) own_w = w[t];
@@ -246,10 +248,12 @@ k_sweep_reg(SweepArgs a)
         const int rank = __popc(vm0 & lt), cnt = __popc(vm0);
         if (valid) s_tok[rank] = make_float4(__int_as_float((int)z0), po0, u0, wt0);
         __syncwarp();
+        uint32_t coming = s_col[(col_at + kRing - 1) & 63];
         float4 tok = s_tok[0];
         // one token: the column of the token kRing - 1 ahead and the next token, then the draw
         auto step = [&](int j, int slot) {
-            load_col(col_at + j + kRing - 1, pv[(slot + kRing - 1) % kRing]);
+            load_col(coming, pv[(slot + kRing - 1) % kRing]);
+            coming = s_col[(col_at + j + kRing) & 63];
             const float4 cur = tok;
             tok = s_tok[j + 1];
             draw(cur, j, pv[slot]);
@@ -262,7 +266,7 @@ k_sweep_reg(SweepArgs a)
             const int count = end - j;
             if (!primed) {
 #pragma unroll
-                for (int q = 0; q < kRing - 1; ++q) load_col(col_at + j + q, pv[q]);
+                for (int q = 0; q < kRing - 1; ++q) load_col(s_col[(col_at + j + q) & 63], pv[q]);
             }
 #pragma unroll 1
             for (; j + kRing <= end; j += kRing) {
@@ -288,8 +292,6 @@ k_sweep_reg(SweepArgs a)
                         int32_t* col = a.nkw_next + (uint64_t)w0 * K;
                         atomicSub(col + z0, 1);
                         atomicAdd(col + znew, 1);
-                        atomicSub(&s_dnk[z0], 1);
-                        atomicAdd(&s_dnk[znew], 1);
                         if (SPLIT && dlt) {
                             atomicSub(&dlt[z0], 1);
                             atomicAdd(&dlt[znew], 1);
@@ -398,7 +400,11 @@ k_sweep_reg(SweepArgs a)
 #pragma unroll
                 for (int t = 0; t < T; ++t) {
                     const int k = topic_of(t);
-                    if (k < K) grow[k] = cn[t];
+                    if (k < K) {
+                        const int change = cn[t] - grow[k];
+                        if (change) atomicAdd(&s_dnk[k], change);
+                        grow[k] = cn[t];
+                    }
                 }
             }
         }
@@ -430,7 +436,13 @@ k_sweep_reg(SweepArgs a)
 #pragma unroll
         for (int t = 0; t < T; ++t) {
             const int k = topic_of(t);
-            if (k < K) grow[k] = (CT)fn[t];
+            if (k < K) {
+                if constexpr (!WT) {
+                    const int change = (int)fn[t] - grow[k];
+                    if (change) atomicAdd(&s_dnk[k], change);
+                }
+                grow[k] = (CT)fn[t];
+            }
         }
     }
     if (!WT) {
