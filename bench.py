@@ -49,7 +49,7 @@ def bytes_per_sweep(N, K, V):
     return N * (4 * K + 16) + 8 * K * V + 4 * (V + 1) + 8 * K
 
 
-# DRAM bytes of one sweep measured by ncu outside the bench (dram__bytes_read.sum +
+# DRAM bytes of one sweep of k_sweep_doc (which ran K = 1000 before k_sweep_wide) measured by ncu outside the bench (dram__bytes_read.sum +
 # dram__bytes_write.sum), keyed by config: shown beside the roofline as the
 # capture it came from; the bench itself measures no DRAM traffic, so its
 # roofline.traffic stays null.
@@ -852,8 +852,8 @@ def main():
                        "optim_interval": 0},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "k_sweep_doc", "kernel_ms": kernel_ms, "alg_bytes_per_launch": alg,
-                         "per": "one sweep = all k_sweep_doc + k_phi_copy launches of the document groups",
+                         "kernel": "training sweep", "kernel_ms": kernel_ms, "alg_bytes_per_launch": alg,
+                         "per": "one sweep = all sweep-kernel and k_phi_copy launches of the document groups",
                          "traffic_ncu": NCU_TRAFFIC.get(args.config) if args.tw == "one" else None,
                          "peak_source": peak_kind},
             "e2e": e2e_obj,

@@ -46,11 +46,11 @@ namespace {
 
 using namespace tmtk;
 constexpr int kSweepWarps = 8;           // warps per sweep block
-// The 16-bit-row kernels (variant 2): 5 warps a block, 5 blocks/SM.  At 8
+// k_sweep_doc's 16-bit-row kernels (variant 1): 5 warps a block, 5 blocks/SM.  At 8
 // warps x 4 blocks the token loop gets 64 registers and spills (spilled
 // registers come back from L2: the resident warps' columns keep L1 from
 // holding them); smaller blocks also leave L1 more of the SM's 256 KB.
-// Measured at k = 1000 (ms per sweep): 8 x 4 101.1 (before alpha moved to
+// Measured at k = 1000, which k_sweep_wide has taken over (ms per sweep): 8 x 4 101.1 (before alpha moved to
 // shared memory; 101.9 after, spilling), 7 x 4 97.6, 6 x 4 92.4,
 // 5 x 4 94.7, 4 x 6 92.7, 4 x 7 97.1, 3 x 8 98.0, 5 x 5 91.4.
 constexpr int kRow16Warps = 5;
@@ -75,8 +75,8 @@ __device__ __forceinline__ float hs_step(float x, int off, float m)
 // 8 stale windows long (at 16 positions per step: 896 tokens; splitting from
 // 421 tokens measured 0.49% lower ll_per_word at the k=100 configuration
 // after 500 sweeps, from 842 tokens 0.03%).  It depends on the corpus only,
-// never on the device or on timing; integer counts with K <= kSplitMaxK (the
-// kernels with phase 1 are built for up to 4 blocks of four topics per lane).
+// never on the device or on timing; integer counts with K <= kSplitMaxK
+// (k_sweep_reg; documents of 2^24 tokens and more in k_sweep_doc).
 // tmt_set_doc_split overrides the threshold and the step.
 constexpr uint32_t kSplitStep = 16;
 constexpr uint32_t kSplitMaxK = 512;
@@ -522,8 +522,9 @@ struct SweepArgs {
 // Topics are dealt to lanes in blocks of four: lane l owns k = 128*j + 4*l + i.
 // Every warp-wide float4 load of a K-vector is one contiguous 512-byte run
 // and shared-memory float4 reads are conflict-free.
-//   CH > 0: at most CH blocks per lane (KP <= 128*CH <= 4096), unrolled.
-//   CH == 0: any K, runtime loops.
+//   CH > 0: at most CH blocks per lane (KP <= 128*CH <= 4096), unrolled (K above
+//       kWideMaxK; k_sweep_reg and k_sweep_wide take the smaller).
+//   CH == 0: any K, runtime loops (K above 4096; documents of 2^24 tokens and more).
 //   WT: weighted counts (TermWeight IDF / PMI): n_dk, n_kw, n_k are floats,
 //       every token carries a weight w, a removal clamps at 0 (updateCnt<true>,
 //       Utils.hpp:132-155) and the count deltas are integers in units of 2^-24.
@@ -760,68 +761,31 @@ k_sweep_doc(SweepArgs a)
                             const int mh = K - 4 * h;
                             const int nh = 4 * (mh >> 7) + min(mh & 127, 4);
                             int found = nh - 1;
-                            if (CH > 0 && CH <= 2) {
-                                // at most 8 topics: lane h forms their Hillis-Steele prefix sums
-                                // (the warp-wide scan's order) from the weights in its registers
+                            // 32 at a time
+                            if (kScratch) {
+                                // lane h's column blocks into the warp's scratch (t-th topic at t)
                                 if (lane == h) {
-                                    float c[4 * CHR];
     #pragma unroll
-                                    for (int jj = 0; jj < CHR; ++jj) {
-                                        const float4 A4 = jj < nch ? *reinterpret_cast<const float4*>(rowf + 128 * jj + 4 * h)
-                                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
-                                        const float av[4] = { A4.x, A4.y, A4.z, A4.w };
-                                        const float pw[4] = { pv[jj].x, pv[jj].y, pv[jj].z, pv[jj].w };
-    #pragma unroll
-                                        for (int i = 0; i < 4; ++i) {
-                                            const int t = 4 * jj + i;
-                                            const int k = 128 * jj + 4 * h + i;
-                                            c[t] = t < nh ? (k == zo ? __fmul_rn(Ao, phi_own) : __fmul_rn(av[i], pw[i])) : 0.f;
-                                        }
-                                    }
-    #pragma unroll
-                                    for (int off = 1; off < 4 * CHR; off <<= 1) {
-    #pragma unroll
-                                        for (int t = 4 * CHR - 1; t >= off; --t) c[t] = __fadd_rn(c[t], c[t - off]);
-                                    }
-                                    bool hit = false;
-    #pragma unroll
-                                    for (int t = 0; t < 4 * CHR; ++t) {
-                                        if (!hit && t < nh && r < __fadd_rn(Eh, c[t])) {
-                                            found = t;
-                                            hit = true;
-                                        }
-                                    }
+                                    for (int jj = 0; jj < CHR; ++jj)
+                                        if (jj < nch) *reinterpret_cast<float4*>(s_xs + 4 * (CHR * warp + jj)) = pv[jj];
                                 }
-                                found = __shfl_sync(FULL, found, h);
-                            } else {
-                                // 32 at a time; up to 16 topics (CH == 4) a 4-step scan gives the
-                                // same prefix values
-                                constexpr int kSteps2 = CH == 4 ? 4 : 5;
-                                if (kScratch) {
-                                    // lane h's column blocks into the warp's scratch (t-th topic at t)
-                                    if (lane == h) {
-    #pragma unroll
-                                        for (int jj = 0; jj < CHR; ++jj)
-                                            if (jj < nch) *reinterpret_cast<float4*>(s_xs + 4 * (CHR * warp + jj)) = pv[jj];
-                                    }
-                                    __syncwarp();
-                                }
-                                float carry = 0.f;
-                                for (int mm = 0; mm < nh; mm += 32) {
-                                    const int t = mm + lane;
-                                    const int k = 128 * (t >> 2) + 4 * h + (t & 3);
-                                    float x2 = 0.f;
-                                    // rowf[zo] reads 0 until the draw: fma(sel, phi_own, 0 * phi) is
-                                    // Ao * phi_own at zo and fma(0, phi_own, p) == p elsewhere
-                                    if (t < nh)
-                                        x2 = __fmaf_rn(k == zo ? Ao : 0.f, phi_own,
-                                                       __fmul_rn(rowf[k], kScratch ? s_xs[4 * CHR * warp + t] : __ldg(ph + k)));
-                                    x2 = scan_n(x2, kSteps2);
-                                    const unsigned mb =
-                                        __ballot_sync(FULL, t < nh && r < __fadd_rn(Eh, __fadd_rn(carry, x2)));
-                                    if (mb) { found = mm + __ffs(mb) - 1; break; }
-                                    carry = __fadd_rn(carry, __shfl_sync(FULL, x2, 31));
-                                }
+                                __syncwarp();
+                            }
+                            float carry = 0.f;
+                            for (int mm = 0; mm < nh; mm += 32) {
+                                const int t = mm + lane;
+                                const int k = 128 * (t >> 2) + 4 * h + (t & 3);
+                                float x2 = 0.f;
+                                // rowf[zo] reads 0 until the draw: fma(sel, phi_own, 0 * phi) is
+                                // Ao * phi_own at zo and fma(0, phi_own, p) == p elsewhere
+                                if (t < nh)
+                                    x2 = __fmaf_rn(k == zo ? Ao : 0.f, phi_own,
+                                                   __fmul_rn(rowf[k], kScratch ? s_xs[4 * CHR * warp + t] : __ldg(ph + k)));
+                                x2 = scan32(x2);
+                                const unsigned mb =
+                                    __ballot_sync(FULL, t < nh && r < __fadd_rn(Eh, __fadd_rn(carry, x2)));
+                                if (mb) { found = mm + __ffs(mb) - 1; break; }
+                                carry = __fadd_rn(carry, __shfl_sync(FULL, x2, 31));
                             }
                             znew = 128 * (found >> 2) + 4 * h + (found & 3);
                         }
@@ -1816,7 +1780,7 @@ void launch_sweep_t(tmt_handle* h, const SweepArgs& a, const SweepShape& sh)
     launch_check(h);
 }
 
-// Variants (identical results, different speed): 0 = the document row in
+// k_sweep_doc's variants (K > kWideMaxK; identical results, different speed): 0 = the document row in
 // shared memory as 32-bit counts, 3 blocks/SM; 1 = the row as 16-bit counts
 // in shared memory (5 warps a block, 5 blocks/SM) or, for documents of
 // 65,536+ tokens, in global memory (4 blocks/SM).  (Measured and dropped:
