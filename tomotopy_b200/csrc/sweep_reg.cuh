@@ -16,7 +16,10 @@
 // tokens at a time, one per lane (words, assignments, uniforms, the own
 // topic's weight, and the count deltas of the tokens that moved), a batch or
 // two ahead of the draws; the words' table columns are loaded kRing - 1 tokens
-// ahead.
+// ahead.  (Products with a 0/1 vector in place of the own topic's selects, and split
+// merges through per-warp buffers in place of shared-memory atomics, measured slower.)
+// 10 sweeps, k_sweep_doc before and this kernel: K = 20, 1.5M tokens 13.5 -> 5.2 ms;
+// K = 100, 27.5M tokens 93 -> 52.5 ms; IDF weights, K = 200, 8M tokens 137 -> 57 ms.
 
 // (counts are held as floats: exact below 2^24 tokens a document, above which
 // the launch takes k_sweep_doc)
