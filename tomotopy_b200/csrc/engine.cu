@@ -1481,9 +1481,12 @@ struct tmt_handle {
     double* d_llv = nullptr;         // tmt_ll output (2)
     double* d_partials = nullptr;
     uint32_t n_partials = 0;
-    // counts set from outside (set_counts): the largest of n_kw (2^32 - 1: some may be
-    // negative); else n_kw is bounded by n_k
-    uint64_t set_max = 0;
+    // counts set from outside (set_counts): sweeps move tokens on and off cells that may
+    // never have held them, so n_k does not bound n_kw, which may be negative
+    bool counts_set = false;
+    // the largest of n_kw (negative ones as large), while no sweep or call has changed it
+    bool kw_max_known = false;
+    uint32_t kw_max = 0;
     double* d_ll = nullptr;          // ll history for one train() call (2 per point)
     uint32_t ll_cap = 0;
     float* d_dg_points = nullptr;
@@ -2429,7 +2432,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
         }
         h->release();
         h->uploaded = false;
-        h->set_max = 0;
+        h->counts_set = h->kw_max_known = false;
         h->D = D;
         h->N_all = n_all;
         h->global_step = 0;
@@ -2780,6 +2783,7 @@ tmt_status tmt_train(tmt_handle* h, uint32_t iters, uint32_t ll_every, double* l
             ++runs;
             in_run = false;
         };
+        h->kw_max_known = false;
         CK(cudaEventRecord(h->tev0, h->stream));
         for (uint32_t i = 0; i < iters; ++i) {
             if (use_graphs && h->tuned >= 0) {
@@ -2926,15 +2930,10 @@ tmt_status tmt_set_counts(tmt_handle* h, const int32_t* n_kw, const int32_t* n_k
         if (!n_kw || !n_k) throw ArgError("n_kw / n_k is NULL");
         if (h->weighted) throw StateError("set_counts takes integer counts; this corpus has weighted counts");
         const uint64_t kv = (uint64_t)h->cfg.K * h->cfg.V;
+        h->counts_set = true;
+        h->kw_max_known = false;
         h2d(h, h->d_nkw[h->cur], n_kw, kv * sizeof(int32_t));
         CK(cudaMemcpyAsync(h->d_nk[h->cur], n_k, h->cfg.K * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemsetAsync(h->d_counter, 0, sizeof(uint32_t), h->stream));
-        k_max_count<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_nkw[h->cur], kv, h->d_counter);
-        launch_check(h);
-        uint32_t mx = 0;
-        CK(cudaMemcpyAsync(&mx, h->d_counter, sizeof(mx), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        h->set_max = std::max<uint64_t>(1, mx);
         CK(cudaStreamSynchronize(h->stream));
     });
 }
@@ -3302,10 +3301,17 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         CK(cudaMemcpyAsync(h->alpha.data(), h->d_alpha, K * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
         std::vector<int32_t> nk(K);                // (float bits when weighted)
         CK(cudaMemcpyAsync(nk.data(), h->d_nk[h->cur], K * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        const bool scan = h->counts_set && !h->kw_max_known;
+        if (scan) {
+            CK(cudaMemsetAsync(B.counter, 0, sizeof(uint32_t), h->stream));
+            k_max_count<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_nkw[h->cur], (uint64_t)K * h->cfg.V, B.counter);
+            launch_check(h);
+            CK(cudaMemcpyAsync(&h->kw_max, B.counter, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+        }
         CK(cudaStreamSynchronize(h->stream));
-        // the largest count with a document's tokens added (integer counts; after
-        // set_counts training may have moved up to N tokens onto a cell)
-        uint64_t longest = 0, most = h->set_max ? h->set_max + h->N : 0;
+        if (scan) h->kw_max_known = true;
+        // the largest count with a document's tokens added (integer counts)
+        uint64_t longest = 0, most = h->counts_set ? h->kw_max : 0;
         for (uint64_t d = 0; d < D; ++d) longest = std::max(longest, doc_off[d + 1] - doc_off[d]);
         for (uint32_t k = 0; k < K; ++k) most = std::max<uint64_t>(most, (uint32_t)nk[k]);
         std::vector<float> acum(K);
