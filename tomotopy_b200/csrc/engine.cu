@@ -2267,8 +2267,9 @@ void do_ll(tmt_handle* h, double* d_out)
         k_ll_final<<<1, 256, 0, h->stream>>>(h->d_partials, h->n_partials, reinterpret_cast<const float*>(h->d_nk[0]),
                                              K, veta, d_out, h->d_esum);
     } else {
-        // the tables lie in the alpha optimiser's partial sums, which are free here: as
-        // many document rows as an eighth of them hold, the rest to the others
+        // the tables lie in the alpha optimiser's partial sums, which are free here: half
+        // of them for the document rows, a quarter each for the others (none where the
+        // partial sums are fewer than four)
         const uint64_t rows = h->n_rows ? h->n_rows : h->D, room = (uint64_t)h->n_apart * K;
         LlTab t{};
         t.nd = (uint32_t)std::min<uint64_t>(1024, h->n_apart / 2);
@@ -2279,7 +2280,7 @@ void do_ll(tmt_handle* h, double* d_out)
         t.len = t.word + t.nw;
         // (not for states whose counts are fewer than the tables' entries)
         const uint64_t entries = (uint64_t)t.nd * K + t.nw + t.nl;
-        const bool use_tab = rows * K + (uint64_t)K * h->cfg.V >= 4 * entries;
+        const bool use_tab = entries && rows * K + (uint64_t)K * h->cfg.V >= 4 * entries;
         const double lg_eta = std::lgamma(eta);
         if (use_tab) {
             k_ll_tab<<<(uint32_t)std::min<uint64_t>((entries + 255) / 256, (uint64_t)h->num_sms * 8), 256, 0, h->stream>>>(
