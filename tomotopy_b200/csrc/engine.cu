@@ -1484,7 +1484,7 @@ struct tmt_handle {
     // counts set from outside (set_counts): sweeps move tokens on and off cells that may
     // never have held them, so n_k does not bound n_kw, which may be negative
     bool counts_set = false;
-    // the largest of n_kw (negative ones as large), while no sweep or call has changed it
+    // the largest of n_kw (k_max_count), while no sweep or call has changed it
     bool kw_max_known = false;
     uint32_t kw_max = 0;
     double* d_ll = nullptr;          // ll history for one train() call (2 per point)
@@ -2425,7 +2425,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
             for (uint64_t i = 0; i < n_all; ++i) {
                 if (wid[i] >= V) continue;
                 const float w = weights[i];
-                if (!(w >= 0.f) || !(w <= 65536.f))
+                if (!(w >= 0.f) || !(w <= (float)kMaxTokenWeight))
                     throw ArgError("token weight " + std::to_string(i) + " is negative, too large or not finite");
                 total += (double)w;
             }
@@ -3021,6 +3021,7 @@ tmt_status tmt_set_counts_f32(tmt_handle* h, const float* n_kw, const float* n_k
             if (!(n_kw[i] >= 0.f) || !std::isfinite(n_kw[i])) throw ArgError("n_kw holds a negative or non-finite value");
         for (uint32_t k = 0; k < h->cfg.K; ++k)
             if (!(n_k[k] >= 0.f) || !std::isfinite(n_k[k])) throw ArgError("n_k holds a negative or non-finite value");
+        h->kw_max_known = false;
         h2d(h, h->d_nkw[0], n_kw, kv * sizeof(float));
         CK(cudaMemcpyAsync(h->d_nk[0], n_k, h->cfg.K * sizeof(float), cudaMemcpyHostToDevice, h->stream));
         CK(cudaStreamSynchronize(h->stream));
@@ -3261,7 +3262,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
                 sorted[i] = pw[i].first;
                 wsorted[i] = pw[i].second;
                 if (sorted[i] >= h->cfg.V) continue;
-                if (!(wsorted[i] >= 0.f) || !(wsorted[i] <= 65536.f))
+                if (!(wsorted[i] >= 0.f) || !(wsorted[i] <= (float)kMaxTokenWeight))
                     throw ArgError("token weight " + std::to_string(i) + " is negative, too large or not finite");
             }
             for (uint64_t d = 0; d < D; ++d)
@@ -3302,7 +3303,9 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         CK(cudaMemcpyAsync(h->alpha.data(), h->d_alpha, K * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
         std::vector<int32_t> nk(K);                // (float bits when weighted)
         CK(cudaMemcpyAsync(nk.data(), h->d_nk[h->cur], K * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-        const bool scan = h->counts_set && !h->kw_max_known;
+        // n_k bounds n_kw unless counts were set; of weighted counts only roughly (a
+        // removal clamps at 0)
+        const bool look = h->counts_set || h->weighted, scan = look && !h->kw_max_known;
         if (scan) {
             CK(cudaMemsetAsync(B.counter, 0, sizeof(uint32_t), h->stream));
             k_max_count<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_nkw[h->cur], (uint64_t)K * h->cfg.V, B.counter);
@@ -3311,10 +3314,10 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         }
         CK(cudaStreamSynchronize(h->stream));
         if (scan) h->kw_max_known = true;
-        // the largest count with a document's tokens added (integer counts)
-        uint64_t longest = 0, most = h->counts_set ? h->kw_max : 0;
+        uint64_t longest = 0;
+        uint32_t most = look ? h->kw_max : 0;
         for (uint64_t d = 0; d < D; ++d) longest = std::max(longest, doc_off[d + 1] - doc_off[d]);
-        for (uint32_t k = 0; k < K; ++k) most = std::max<uint64_t>(most, (uint32_t)nk[k]);
+        for (uint32_t k = 0; k < K; ++k) most = std::max(most, (uint32_t)nk[k]);
         std::vector<float> acum(K);
         float sf = 0.f;
         double sd = 0;
@@ -3370,7 +3373,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         a.esum = h->d_esum;
         a.pcum = h->d_prior_cum;
         a.ecum = h->d_cum_eta;
-        a.small_counts = h->weighted || most + longest < (1u << 23);   // (weighted counts are never negative)
+        a.count_max = count_bound(most, h->weighted) + (double)longest * (h->weighted ? kMaxTokenWeight : 1.0);
         launch_infer(a, h->num_sms, h->stream);
         ++h->launches;
         if (theta) d2h(h, theta, B.theta, D * (uint64_t)K * sizeof(float));

@@ -19,6 +19,7 @@
 #pragma once
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 #include "common.cuh"
 #include "philox.cuh"
@@ -65,10 +66,22 @@ struct InferArgs {
     const float* esum;
     const float* pcum;
     const float* ecum;
-    // no n_k (nor n_kw) is negative, and with a document's tokens added none
-    // reaches 2^23 (weighted counts: only the former)
-    bool small_counts;
+    // no n_k or n_kw with a document's tokens added is larger; infinity if one may be
+    // negative or not a number (count_bound)
+    double count_max;
 };
+
+// The bound on counts of which k_max_count found `bits` the largest.
+inline double count_bound(uint32_t bits, bool weighted)
+{
+    if (!weighted) return bits > 0x7FFFFFFFu ? INFINITY : (double)bits;
+    if (bits > 0x7F800000u) return INFINITY;
+    float f;
+    std::memcpy(&f, &bits, sizeof(f));
+    return (double)f;
+}
+
+constexpr double kMaxTokenWeight = 65536.0;      // what the callers accept
 
 // A finished document's theta and FP64 ll over the cells it touched.  dlen: its
 // length (weight sum); own: K zeroed ints, zeroed again on return; count(k): its n_dk.
@@ -487,10 +500,12 @@ inline void launch_infer_reg_g(const InferArgs& a, int num_sms, cudaStream_t st)
     // The fast modes' conditions: scalar eta, counts exact in to_f, denominators in
     // recip's range.  (Their general forms cost a draw at k = 100 about 50 of 450
     // cycles.)  Element loads where columns are not 16-byte aligned.
-    // (No weight or sum of weights can overflow: A B R below 1e36 / K.)
-    const double most = WT ? 549755813888.0 : 8388608.0;
+    // (No weight or sum of weights can overflow: A B R below 1e36 / K.  With V eta at
+    // most 1e30 this also keeps weighted counts below 1e31, inside recip's range.)
+    const double most = WT ? a.count_max : 8388608.0;
     const bool finite = (most + (double)a.asum_f) * (most + (double)a.eta) < 1e32 * (double)a.veta;
-    if (a.pidx || !a.small_counts || !finite || !(a.veta >= 1e-30f && a.veta <= 1e30f))
+    const bool exact = WT || a.count_max < 8388608.0;
+    if (a.pidx || !exact || !finite || !(a.veta >= 1e-30f && a.veta <= 1e30f))
         launch_infer_reg_t<CH, 5, WT, 2>(a, num_sms, st);
     else if (a.K & 3) launch_infer_reg_t<CH, STEPS, WT, 1>(a, num_sms, st);
     else launch_infer_reg_t<CH, STEPS, WT, 0>(a, num_sms, st);
@@ -508,7 +523,8 @@ inline void launch_infer_reg(const InferArgs& a, int num_sms, cudaStream_t st)
     else launch_infer_reg_g<8, 5, WT>(a, num_sms, st);
 }
 
-// the largest of n counts, negative ones as large (out must be 0 before)
+// the largest of n counts, or of non-negative floats by their bits; negative ones (and
+// NaN) as larger than all others (out must be 0 before)
 static __global__ void k_max_count(const int32_t* __restrict__ c, uint64_t n, uint32_t* __restrict__ out)
 {
     uint32_t m = 0;

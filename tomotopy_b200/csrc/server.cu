@@ -167,7 +167,7 @@ struct Model {
     float* d_pcum = nullptr;
     float* d_ecum = nullptr;
     bool used = false;                  // a request was submitted: the model is frozen
-    uint64_t count_max = 0;             // no n_k or n_kw is larger (2^32 - 1: some may be negative)
+    double count_max = 0;               // no n_k or n_kw is larger (infinity: some may be negative)
     bool weighted = false;              // float counts (TermWeight IDF / PMI); requests carry weights
 };
 
@@ -395,7 +395,7 @@ bool server_step(tmt_server* s)
         a.esum = m->d_esum;
         a.pcum = m->d_pcum;
         a.ecum = m->d_ecum;
-        a.small_counts = m->count_max + s->cfg.max_doc_len < (1u << 23);
+        a.count_max = m->count_max + (double)s->cfg.max_doc_len * (m->weighted ? kMaxTokenWeight : 1.0);
         // every request of a model shares the draw key base; the per-request seed is folded in below
         a.key = 0;
         // requests may carry different seeds: launch per distinct seed (usually one)
@@ -632,18 +632,13 @@ tmt_status add_model_impl(tmt_server* s, uint32_t K, uint32_t V, const float* al
         if ((uint64_t)K * V)
             CK(cudaMemcpy(m->d_nkw, n_kw, (uint64_t)K * V * 4, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(m->d_nk, n_k, K * 4, cudaMemcpyHostToDevice));
-        if (weighted) {
-            for (uint32_t k = 0; k < K; ++k)
-                if (!(static_cast<const float*>(n_k)[k] >= 0.f)) m->count_max = 0xFFFFFFFFu;
-        } else {
-            uint32_t mx = 0;
-            CK(cudaMemset(m->d_counter, 0, sizeof(uint32_t)));
-            k_max_count<<<1184, 256>>>(m->d_nkw, (uint64_t)K * V, m->d_counter);
-            k_max_count<<<1, 256>>>(m->d_nk, K, m->d_counter);
-            CK(cudaGetLastError());
-            CK(cudaMemcpy(&mx, m->d_counter, sizeof(mx), cudaMemcpyDeviceToHost));
-            m->count_max = mx;
-        }
+        uint32_t mx = 0;
+        CK(cudaMemset(m->d_counter, 0, sizeof(uint32_t)));
+        k_max_count<<<1184, 256>>>(m->d_nkw, (uint64_t)K * V, m->d_counter);
+        k_max_count<<<1, 256>>>(m->d_nk, K, m->d_counter);
+        CK(cudaGetLastError());
+        CK(cudaMemcpy(&mx, m->d_counter, sizeof(mx), cudaMemcpyDeviceToHost));
+        m->count_max = count_bound(mx, weighted);
         CK(cudaMemcpy(m->d_alpha, alpha, K * sizeof(float), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(m->d_acum, acum.data(), K * sizeof(float), cudaMemcpyHostToDevice));
     } catch (const OomError&) {
@@ -665,7 +660,7 @@ tmt_status make_request(tmt_server* s, const uint32_t* wid, const float* wts, ui
     if (wts) {
         std::vector<std::pair<uint32_t, float>> pw(len);
         for (uint64_t i = 0; i < len; ++i) {
-            if (!(wts[i] >= 0.f) || !(wts[i] <= 65536.f)) return TMT_ERR_INVALID_ARGUMENT;
+            if (!(wts[i] >= 0.f) || !(wts[i] <= (float)kMaxTokenWeight)) return TMT_ERR_INVALID_ARGUMENT;
             pw[i] = { wid[i], wts[i] };
         }
         std::stable_sort(pw.begin(), pw.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
