@@ -1484,9 +1484,9 @@ struct tmt_handle {
     // counts set from outside (set_counts): sweeps move tokens on and off cells that may
     // never have held them, so n_k does not bound n_kw, which may be negative
     bool counts_set = false;
-    // the largest of n_kw (k_max_count), while no sweep or call has changed it
-    bool kw_max_known = false;
-    uint32_t kw_max = 0;
+    // the largest count (k_max_count), while no sweep or call has changed it
+    bool max_known = false;
+    uint32_t count_max = 0;
     double* d_ll = nullptr;          // ll history for one train() call (2 per point)
     uint32_t ll_cap = 0;
     float* d_dg_points = nullptr;
@@ -1502,6 +1502,7 @@ struct tmt_handle {
         float* acum = nullptr;
         uint32_t* counter = nullptr;
         uint32_t* work = nullptr;        // documents, longest first
+        uint64_t cap_work = 0;
         float* wt = nullptr;
         uint64_t cap_wt = 0;
     } inf;
@@ -2433,7 +2434,7 @@ tmt_status upload_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_o
         }
         h->release();
         h->uploaded = false;
-        h->counts_set = h->kw_max_known = false;
+        h->counts_set = h->max_known = false;
         h->D = D;
         h->N_all = n_all;
         h->global_step = 0;
@@ -2784,7 +2785,7 @@ tmt_status tmt_train(tmt_handle* h, uint32_t iters, uint32_t ll_every, double* l
             ++runs;
             in_run = false;
         };
-        h->kw_max_known = false;
+        h->max_known = false;
         CK(cudaEventRecord(h->tev0, h->stream));
         for (uint32_t i = 0; i < iters; ++i) {
             if (use_graphs && h->tuned >= 0) {
@@ -2932,7 +2933,7 @@ tmt_status tmt_set_counts(tmt_handle* h, const int32_t* n_kw, const int32_t* n_k
         if (h->weighted) throw StateError("set_counts takes integer counts; this corpus has weighted counts");
         const uint64_t kv = (uint64_t)h->cfg.K * h->cfg.V;
         h->counts_set = true;
-        h->kw_max_known = false;
+        h->max_known = false;
         h2d(h, h->d_nkw[h->cur], n_kw, kv * sizeof(int32_t));
         CK(cudaMemcpyAsync(h->d_nk[h->cur], n_k, h->cfg.K * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
         CK(cudaStreamSynchronize(h->stream));
@@ -3021,7 +3022,7 @@ tmt_status tmt_set_counts_f32(tmt_handle* h, const float* n_kw, const float* n_k
             if (!(n_kw[i] >= 0.f) || !std::isfinite(n_kw[i])) throw ArgError("n_kw holds a negative or non-finite value");
         for (uint32_t k = 0; k < h->cfg.K; ++k)
             if (!(n_k[k] >= 0.f) || !std::isfinite(n_k[k])) throw ArgError("n_k holds a negative or non-finite value");
-        h->kw_max_known = false;
+        h->max_known = false;
         h2d(h, h->d_nkw[0], n_kw, kv * sizeof(float));
         CK(cudaMemcpyAsync(h->d_nk[0], n_k, h->cfg.K * sizeof(float), cudaMemcpyHostToDevice, h->stream));
         CK(cudaStreamSynchronize(h->stream));
@@ -3279,7 +3280,6 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
             B.doc_off = h->dalloc<uint64_t>(D + 1);
             B.keys = h->dalloc<uint64_t>(D);
             B.ll = h->dalloc<double>(D);
-            B.work = h->dalloc<uint32_t>(D);
             B.cap_docs = D;
         }
         if (D * K > B.cap_theta) {
@@ -3301,23 +3301,24 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         }
         // alpha of the current state (after any optimisation)
         CK(cudaMemcpyAsync(h->alpha.data(), h->d_alpha, K * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-        std::vector<int32_t> nk(K);                // (float bits when weighted)
-        CK(cudaMemcpyAsync(nk.data(), h->d_nk[h->cur], K * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-        // n_k bounds n_kw unless counts were set; of weighted counts only roughly (a
-        // removal clamps at 0)
-        const bool look = h->counts_set || h->weighted, scan = look && !h->kw_max_known;
-        if (scan) {
+        // the largest count: n_k bounds n_kw unless counts were set (and weighted ones only
+        // roughly, since a removal clamps at 0), the tokens n_k
+        const bool look = h->counts_set || h->weighted;
+        const bool few = !look && h->world == 1 && h->N < (1u << 22);
+        if (!few && !h->max_known) {
             CK(cudaMemsetAsync(B.counter, 0, sizeof(uint32_t), h->stream));
-            k_max_count<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_nkw[h->cur], (uint64_t)K * h->cfg.V, B.counter);
+            if (look) {
+                k_max_count<<<h->num_sms * 8, 256, 0, h->stream>>>(h->d_nkw[h->cur], (uint64_t)K * h->cfg.V, B.counter);
+                launch_check(h);
+            }
+            k_max_count<<<1, 256, 0, h->stream>>>(h->d_nk[h->cur], K, B.counter);
             launch_check(h);
-            CK(cudaMemcpyAsync(&h->kw_max, B.counter, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaMemcpyAsync(&h->count_max, B.counter, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
         }
         CK(cudaStreamSynchronize(h->stream));
-        if (scan) h->kw_max_known = true;
+        if (!few) h->max_known = true;
         uint64_t longest = 0;
-        uint32_t most = look ? h->kw_max : 0;
         for (uint64_t d = 0; d < D; ++d) longest = std::max(longest, doc_off[d + 1] - doc_off[d]);
-        for (uint32_t k = 0; k < K; ++k) most = std::max(most, (uint32_t)nk[k]);
         std::vector<float> acum(K);
         float sf = 0.f;
         double sd = 0;
@@ -3326,14 +3327,28 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         CK(cudaMemcpyAsync(B.doc_off, doc_off, (D + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
         h2d(h, B.words, sorted.data(), n_all * sizeof(uint32_t));
         if (weights) h2d(h, B.wt, wsorted.data(), n_all * sizeof(float));
-        // longest documents first: a document is one warp's chain, and a long one
-        // taken up last would run on alone
-        std::vector<uint32_t> work(D);
-        std::iota(work.begin(), work.end(), 0u);
-        std::stable_sort(work.begin(), work.end(), [&](uint32_t x, uint32_t y) {
-            return doc_off[x + 1] - doc_off[x] > doc_off[y + 1] - doc_off[y];
-        });
-        CK(cudaMemcpyAsync(B.work, work.data(), D * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        // Longest documents first (to a 4,096th of the longest): a document is one warp's
+        // chain, and a long one taken up last would run on alone.  Not where every document
+        // starts at once, nor where the longest is at most twice the mean or short beside
+        // what each of ~16 warps an SM is given: there the order only costs its making and its copy.
+        const uint64_t sms = (uint64_t)h->num_sms;
+        std::vector<uint32_t> work;
+        if (D > sms * kInferRegWarps && longest * D > 2 * n_all && longest * sms * 16 * 8 > n_all) {
+            constexpr uint32_t kBuckets = 4096;
+            uint32_t shift = 0;
+            while ((longest >> shift) >= kBuckets) ++shift;
+            auto bucket = [&](uint64_t d) { return kBuckets - 1 - (uint32_t)((doc_off[d + 1] - doc_off[d]) >> shift); };
+            uint32_t first[kBuckets + 1] = {};
+            for (uint64_t d = 0; d < D; ++d) ++first[bucket(d) + 1];
+            for (uint32_t i = 0; i < kBuckets; ++i) first[i + 1] += first[i];
+            work.resize(D);
+            for (uint64_t d = 0; d < D; ++d) work[first[bucket(d)]++] = (uint32_t)d;
+            if (D > B.cap_work) {
+                B.work = h->dalloc<uint32_t>(D);
+                B.cap_work = D;
+            }
+            CK(cudaMemcpyAsync(B.work, work.data(), D * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        }
         if (doc_keys) CK(cudaMemcpyAsync(B.keys, doc_keys, D * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(B.acum, acum.data(), K * sizeof(float), cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(B.counter, 0, sizeof(uint32_t), st));
@@ -3364,7 +3379,7 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         a.ndk = nullptr;
         a.theta = B.theta;
         a.ll = B.ll;
-        a.work = B.work;
+        a.work = work.empty() ? nullptr : B.work;
         a.n_work = (uint32_t)D;
         a.counter = B.counter;
         a.wt = weights ? B.wt : nullptr;
@@ -3373,7 +3388,8 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         a.esum = h->d_esum;
         a.pcum = h->d_prior_cum;
         a.ecum = h->d_cum_eta;
-        a.count_max = count_bound(most, h->weighted) + (double)longest * (h->weighted ? kMaxTokenWeight : 1.0);
+        a.count_max = (few ? (double)h->N : count_bound(h->count_max, h->weighted)) +
+                      (double)longest * (h->weighted ? kMaxTokenWeight : 1.0);
         launch_infer(a, h->num_sms, h->stream);
         ++h->launches;
         if (theta) d2h(h, theta, B.theta, D * (uint64_t)K * sizeof(float));
