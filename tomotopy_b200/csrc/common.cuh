@@ -43,6 +43,19 @@ __device__ __forceinline__ float up1_or_0(float x)
     return r;
 }
 
+// 1 / x rounded to nearest, without a branch, for x in [2^-107, 2^104): one Newton step
+// from an approximation within one ulp is exact rounding but for divisors whose
+// mantissa is all ones (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), where it depends on the
+// approximation; on sm_100 it equals __frcp_rn for every mantissa of these
+// exponents (tests/test_recip_gpu.py).
+__device__ __forceinline__ float recip_mid(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.f), y);
+}
+
 __host__ __device__ __forceinline__ uint32_t round4(uint32_t x) { return (x + 3u) & ~3u; }
 
 __device__ __forceinline__ double warp_sum(double x)

@@ -79,23 +79,9 @@ k_infer_reg(InferArgs a)
     auto at = [&](int k) { return kWide ? (k & ~127) | ((k + 4 * (k >> 7)) & 127) : k; };
     const int my4 = 4 * lane;
     auto blk = [&](int jj) { return 128 * jj + (kWide ? ((my4 + 4 * jj) & 127) : my4); };
-    // Reciprocals, rounded to nearest.  In the fast modes the denominators lie in
-    // [V eta, 2^23 + V eta] (weighted: n_k's range above V eta) with V eta in [1e-30,
-    // 1e30]; one Newton step from an approximation within one ulp is then
-    // exact rounding but for divisors whose mantissa is all ones (P. Markstein,
-    // "Computation of elementary functions on the IBM RISC System/6000
-    // processor", IBM J. Res. Dev. 34, 1990), where it depends on the
-    // approximation: compared with __frcp_rn for every mantissa of the exponents
-    // 2^-107 .. 2^103 on sm_100, no difference.  It has no branch.
-    auto recip = [](float x) -> float {
-        if constexpr (GEN) {
-            return __frcp_rn(x);
-        } else {
-            float y;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-            return __fmaf_rn(y, __fmaf_rn(-x, y, 1.f), y);
-        }
-    };
+    // the denominators lie in recip_mid's range in the fast modes (launch_infer_reg_g):
+    // V eta in [1e-30, 1e30] and counts below 1e31 above it
+    auto recip = [](float x) -> float { return GEN ? __frcp_rn(x) : recip_mid(x); };
     // (float)n of a count: in the fast modes below 2^23, where 2^23 + n is exact in
     // the float whose mantissa holds n (the conversion unit does one warp in 8 cycles)
     auto to_f = [](CT n) -> float {
