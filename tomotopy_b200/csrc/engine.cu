@@ -3329,11 +3329,11 @@ tmt_status infer_impl(tmt_handle* h, const uint32_t* wid, const uint64_t* doc_of
         if (weights) h2d(h, B.wt, wsorted.data(), n_all * sizeof(float));
         // Longest documents first (to a 4,096th of the longest): a document is one warp's
         // chain, and a long one taken up last would run on alone.  Not where every document
-        // starts at once, nor where the longest is at most twice the mean or short beside
-        // what each of ~16 warps an SM is given: there the order only costs its making and its copy.
+        // starts at once, all are alike or the longest is short beside what each of ~16 warps
+        // an SM is given: there the order only costs its making and its copy.
         const uint64_t sms = (uint64_t)h->num_sms;
         std::vector<uint32_t> work;
-        if (D > sms * kInferRegWarps && longest * D > 2 * n_all && longest * sms * 16 * 8 > n_all) {
+        if (D > sms * kInferRegWarps && longest * D > n_all && longest * sms * 16 * 8 > n_all) {
             constexpr uint32_t kBuckets = 4096;
             uint32_t shift = 0;
             while ((longest >> shift) >= kBuckets) ++shift;
