@@ -24,6 +24,14 @@
 constexpr uint32_t kInferRegMaxK = 1024;
 constexpr int kInferRegWarps = 4;    // warps (documents) per block: one per SM sub-partition
 
+// resident blocks per SM (registers a thread may use), as many as leave the draws
+// (nearly) without spills and as the arrays' shared memory admits
+template <int CH, int MODE>
+struct InferRegBlocks {
+    static constexpr int value = CH <= 1 ? 5 : CH <= 2 ? 6 : CH <= 4 ? 4 : CH <= 5 ? (MODE == 2 ? 3 : 4)
+                                 : CH <= 7 ? 3 : 2;
+};
+
 //   CH: blocks of four topics per lane (K <= 128 CH); STEPS: steps of the lane scan,
 //       the lanes that hold topics being the first 2^STEPS at most
 //   WT: weighted counts (TermWeight IDF / PMI)
@@ -31,7 +39,7 @@ constexpr int kInferRegWarps = 4;    // warps (documents) per block: one per SM 
 //        1: the fast conditions, columns loaded by the element;
 //        2: any (word priors, counts of 2^23 and more, extreme V eta)
 template <int CH, int STEPS, bool WT, int MODE>
-__global__ void __launch_bounds__(kInferRegWarps * 32, CH <= 1 ? 5 : CH <= 2 ? 6 : CH <= 4 ? 4 : 2)
+__global__ void __launch_bounds__(kInferRegWarps * 32, InferRegBlocks<CH, MODE>::value)
 k_infer_reg(InferArgs a)
 {
     using CT = typename std::conditional<WT, float, int>::type;
@@ -78,6 +86,7 @@ k_infer_reg(InferArgs a)
     // lanes, so that one lane's topics sit in different banks
     auto at = [&](int k) { return kWide ? (k & ~127) | ((k + 4 * (k >> 7)) & 127) : k; };
     const int my4 = 4 * lane;
+    const bool vec = MODE == 0 || (GEN && kWide && (K & 3) == 0);    // 16-byte column loads
     auto blk = [&](int jj) { return 128 * jj + (kWide ? ((my4 + 4 * jj) & 127) : my4); };
     // the denominators lie in recip_mid's range in the fast modes (launch_infer_reg_g):
     // V eta in [1e-30, 1e30] and counts below 1e31 above it
@@ -298,12 +307,14 @@ k_infer_reg(InferArgs a)
         // (a lane's blocks past K are never loaded and stay 0)
         auto load_col = [&](float word, G4 (&g)[CH]) {
             const CT* col = nkw + (uint64_t)(uint32_t)__float_as_int(word) * (uint32_t)K + my4;
+            if (vec) {
 #pragma unroll
-            for (int jj = 0; jj < CH; ++jj) {
-                const int k0 = 128 * jj + my4;
-                if constexpr (MODE == 0) {
-                    if (k0 < K) g[jj] = __ldg(reinterpret_cast<const G4*>(col + 128 * jj));
-                } else {
+                for (int jj = 0; jj < CH; ++jj)
+                    if (128 * jj + my4 < K) g[jj] = __ldg(reinterpret_cast<const G4*>(col + 128 * jj));
+            } else {
+#pragma unroll
+                for (int jj = 0; jj < CH; ++jj) {
+                    const int k0 = 128 * jj + my4;
                     if (k0 < K) g[jj].x = __ldg(col + 128 * jj);
                     if (k0 + 1 < K) g[jj].y = __ldg(col + 128 * jj + 1);
                     if (k0 + 2 < K) g[jj].z = __ldg(col + 128 * jj + 2);
@@ -327,6 +338,13 @@ k_infer_reg(InferArgs a)
                 gb[jj] = ga[jj];
             }
             load_col(tok.w, ga);
+            // the prior column of a word, NULL if it has none
+            auto prior_of = [&](float word) -> const float* {
+                if (!GEN || !a.pidx) return nullptr;
+                const int p = __ldg(a.pidx + (uint32_t)__float_as_int(word));
+                return p >= 0 ? a.pval + (uint64_t)p * K : nullptr;
+            };
+            const float* pe_next = GEN && kWide ? prior_of(tok.w) : nullptr;     // (of the coming token)
             bool in_run = kind_of(tok) == 1;
             {
                 // the first token leaves its topic
@@ -359,6 +377,38 @@ k_infer_reg(InferArgs a)
                 const int zn = min(topic(nt), K - 1);    // the topic the next token leaves (if there is one)
                 const int kind = kind_of(tok);
                 const float u = tok.y, wt = tok.z;
+                // The word's prior column, if any.  With CH > 4 it is looked up a token ahead
+                // and loaded at once (6,000 documents of 80 tokens, 60 sweeps, priors: K = 1000
+                // 57 -> 50 ms); below, the lookup costs more than its latency (K = 100, 64
+                // documents: 10.1 against 11.3 ms).
+                const float* pe = nullptr;
+                if (GEN && !kWide) pe = prior_of(tok.w);
+                float w[T];                          // CH > 4: the etas; then, in pass 1, the weights
+                if constexpr (GEN && kWide) {
+                    pe = pe_next;
+                    pe_next = prior_of(nt.w);
+#pragma unroll
+                    for (int t = 0; t < T; ++t) w[t] = eta;
+                    if (pe && vec) {
+#pragma unroll
+                        for (int jj = 0; jj < CH; ++jj)
+                            if (128 * jj + my4 < K) {
+                                const float4 e = __ldg(reinterpret_cast<const float4*>(pe + 128 * jj + my4));
+                                w[4 * jj] = e.x;
+                                w[4 * jj + 1] = e.y;
+                                w[4 * jj + 2] = e.z;
+                                w[4 * jj + 3] = e.w;
+                            }
+                    } else if (pe) {
+#pragma unroll
+                        for (int t = 0; t < T; ++t)
+                            if (topic_of(t) < K) w[t] = __ldg(pe + topic_of(t));
+                    }
+                }
+                auto ek = [&](int t) -> float {
+                    if constexpr (GEN && kWide) return w[t];
+                    else return GEN && pe && topic_of(t) < K ? __ldg(pe + topic_of(t)) : eta;
+                };
                 // the run's other tokens of the word (zero outside a run)
                 if (CH <= 2 || in_run)
 #pragma unroll
@@ -376,15 +426,9 @@ k_infer_reg(InferArgs a)
                         g[jj].w += o.w;
                     }
                 }
-                const float* pe = nullptr;           // the word's prior column, if any
-                if (GEN && a.pidx) {
-                    const int p = __ldg(a.pidx + (uint32_t)__float_as_int(tok.w));
-                    if (p >= 0) pe = a.pval + (uint64_t)p * K;
-                }
-                auto ek = [&](int t) { return GEN && pe && topic_of(t) < K ? __ldg(pe + topic_of(t)) : eta; };
                 // pass 1: fma chain over this lane's topics; w: A_k for CH <= 4
                 // turned into the weights, above B_k R_k
-                float w[T], s = 0.f;
+                float s = 0.f;
 #pragma unroll
                 for (int jj = 0; jj < CH; ++jj) {
                     const float4 A4 = *reinterpret_cast<const float4*>(s_A + blk(jj));
