@@ -67,7 +67,7 @@ __device__ __forceinline__ float hs_step(float x, int off, float m)
 
 // Long documents: a document of at least split_len tokens (all ids counted)
 // is sampled by a whole block as kSweepWarps slices side by side, merging
-// their n_dk changes every split_step positions (k_sweep_doc, phase 1).  A
+// their n_dk changes every split_step positions (k_sweep_reg, phase 1).  A
 // token then sees up to (kSweepWarps - 1) * split_step of its document's
 // other tokens as of the step's start.  The threshold of a document group is
 // max(8 * (kSweepWarps - 1) * split_step, ceil(tokens / 4096)): documents
@@ -76,7 +76,7 @@ __device__ __forceinline__ float hs_step(float x, int off, float m)
 // 421 tokens measured 0.49% lower ll_per_word at the k=100 configuration
 // after 500 sweeps, from 842 tokens 0.03%).  It depends on the corpus only,
 // never on the device or on timing; integer counts with K <= kSplitMaxK
-// (k_sweep_reg; documents of 2^24 tokens and more in k_sweep_doc).
+// (k_sweep_reg; documents of 2^31 tokens and more in k_sweep_doc).
 // tmt_set_doc_split overrides the threshold and the step.
 constexpr uint32_t kSplitStep = 16;
 constexpr uint32_t kSplitMaxK = 512;
@@ -541,7 +541,7 @@ struct SweepArgs {
 // and shared-memory float4 reads are conflict-free.
 //   CH > 0: at most CH blocks per lane (KP <= 128*CH <= 4096), unrolled (K above
 //       kWideMaxK; k_sweep_reg and k_sweep_wide take the smaller).
-//   CH == 0: any K, runtime loops (K above 4096; documents of 2^24 tokens and more).
+//   CH == 0: any K, runtime loops (K above 4096; K <= 512 with documents of 2^31 tokens and more).
 //   WT: weighted counts (TermWeight IDF / PMI): n_dk, n_kw, n_k are floats,
 //       every token carries a weight w, a removal clamps at 0 (updateCnt<true>,
 //       Utils.hpp:132-155) and the count deltas are integers in units of 2^-24.
@@ -1853,10 +1853,10 @@ void launch_sweep_w(tmt_handle* h, const SweepArgs& b, const SweepShape& sh, uin
 }
 
 // --- k_sweep_reg: K <= kRegMaxK ---
-template <int CH, int STEPS, bool WT, bool SPLIT, bool OPT>
+template <int CH, int STEPS, bool WT, bool SPLIT, bool OPT, bool BIG = false>
 void launch_reg_t(tmt_handle* h, const SweepArgs& a)
 {
-    auto kern = k_sweep_reg<CH, STEPS, WT, SPLIT, OPT>;
+    auto kern = k_sweep_reg<CH, STEPS, WT, SPLIT, OPT, BIG>;
     const uint32_t warps = SPLIT ? kSweepWarps : kRegWarps;
     const uint32_t smem = WT ? 0 : 4 * round4(a.K) * (SPLIT ? 4 : 1);      // at most 8 KB
     int per_sm = 0;
@@ -1879,6 +1879,14 @@ template <int CH, int STEPS>
 void launch_reg_ch(tmt_handle* h, const SweepArgs& a)
 {
     const bool opt = a.arow || a.mask;
+    if (!a.wt && a.max_len >= kRegFloatLen) {
+        // One document of 2^24 + 77 tokens, split, a sweep: K = 20 562 ms against 2,456 in the
+        // general k_sweep_doc (unrolled: 1,422), K = 400 1,445 (2,256 unrolled).  (A scan of all
+        // five steps gives the same sums.)
+        if (a.n_long) launch_reg_t<CH, 5, false, true, true, true>(h, a);
+        else launch_reg_t<CH, 5, false, false, true, true>(h, a);
+        return;
+    }
     if (a.wt) opt ? launch_reg_t<CH, STEPS, true, false, true>(h, a) : launch_reg_t<CH, STEPS, true, false, false>(h, a);
     else if (a.n_long) opt ? launch_reg_t<CH, STEPS, false, true, true>(h, a) : launch_reg_t<CH, STEPS, false, true, false>(h, a);
     else opt ? launch_reg_t<CH, STEPS, false, false, true>(h, a) : launch_reg_t<CH, STEPS, false, false, false>(h, a);

@@ -21,17 +21,16 @@
 // 10 sweeps, k_sweep_doc before and this kernel: K = 20, 1.5M tokens 13.5 -> 5.2 ms;
 // K = 100, 27.5M tokens 93 -> 52.5 ms; IDF weights, K = 200, 8M tokens 137 -> 57 ms.
 
-// (counts are held as floats: exact below 2^24 tokens a document, above which
-// the launch takes k_sweep_doc)
 constexpr uint32_t kRegMaxK = 512;
-constexpr uint64_t kRegMaxLen = 1ull << 24;
+constexpr uint64_t kRegFloatLen = 1ull << 24;    // counts below are exact as floats
+constexpr uint64_t kRegMaxLen = 1ull << 31;      // positions are 32 bits; from here on k_sweep_doc
 constexpr int kRegWarps = 4;         // warps per block without split documents: one per SM sub-partition
 
 // resident blocks per SM (registers a thread may use): as many as leave the
 // token loop without spills (6 blocks of 80 registers with CH = 1 spilled 40 bytes:
 // K = 100, 27.5M tokens, 10 sweeps 59-61 against 55 ms with 5; split documents at
 // 2 blocks of 8 warps spilled 40-140 with CH = 2 and 3: K = 333 26.9 against 25.4 ms)
-template <int CH, bool SPLIT, bool OPT>
+template <int CH, bool SPLIT>
 struct RegBlocks {
     static constexpr int value = SPLIT ? (CH <= 1 ? 2 : 1)
                                        : CH <= 1 ? 5 : CH <= 2 ? 4 : 3;
@@ -44,12 +43,16 @@ struct RegBlocks {
 //   SPLIT: the launch's first n_long documents are sampled a block each in
 //       kSweepWarps slices (see kSplitStep); integer counts
 //   OPT: per-document masks or alphas may be set
-template <int CH, int STEPS, bool WT, bool SPLIT, bool OPT>
-__global__ void __launch_bounds__((SPLIT ? kSweepWarps : kRegWarps) * 32, RegBlocks<CH, SPLIT, OPT>::value)
+//   BIG: documents of kRegFloatLen tokens and more: integer counts are held as integers
+//       (a conversion per topic and draw; as floats they need none)
+template <int CH, int STEPS, bool WT, bool SPLIT, bool OPT, bool BIG>
+__global__ void __launch_bounds__((SPLIT ? kSweepWarps : kRegWarps) * 32, RegBlocks<CH, SPLIT>::value)
 k_sweep_reg(SweepArgs a)
 {
     static_assert(!(SPLIT && WT), "split documents have integer counts");
+    static_assert(!(BIG && WT), "weighted counts are floats");
     using CT = typename std::conditional<WT, float, int>::type;
+    using FT = typename std::conditional<BIG, int, float>::type;
     constexpr int T = 4 * CH;            // topics per lane
     constexpr int kRing = CH <= 2 ? 4 : 2;
     constexpr int kWarps = SPLIT ? kSweepWarps : kRegWarps;
@@ -84,7 +87,8 @@ k_sweep_reg(SweepArgs a)
     const float eta = a.eta, veta = a.veta;
     const uint32_t iter = a.iter_ptr ? *a.iter_ptr : a.iter;
 
-    float fn[T], al[T], mk[OPT ? T : 1]; // counts, alphas, mask (1 / 0) of this lane's topics
+    FT fn[T];                            // counts of this lane's topics
+    float al[T], mk[OPT ? T : 1];        // their alphas, mask (1 / 0)
     auto topic_of = [&](int t) { return 128 * (t >> 2) + 4 * lane + (t & 3); };
     auto load_alpha = [&](const float* alpha) {
 #pragma unroll
@@ -112,7 +116,7 @@ k_sweep_reg(SweepArgs a)
     CT nkw1 = CT(0);
     float ri1 = 0.f, u0 = 0.f, po0 = 0.f;
     // The current document's (or slice's) tokens are [0, len) from token tok0;
-    // positions and lengths are below 2^24 (kRegMaxLen).
+    // positions and lengths are below 2^31 (kRegMaxLen).
     uint64_t tok0 = 0;
     uint32_t col_at = 0, col_end = 0;    // s_col: the current batch's first entry, the next one's end (mod 64)
     unsigned vm1 = 0, vm0 = 0;           // the lanes whose word is sampled
@@ -194,9 +198,9 @@ k_sweep_reg(SweepArgs a)
             const bool own = zr == 128 * (t >> 2) + (t & 3);
             if (own) {
                 if constexpr (WT) fn[t] = fmaxf(__fsub_rn(fn[t], wt), 0.f);
-                else fn[t] = __fsub_rn(fn[t], 1.f);
+                else fn[t] -= FT(1);
             }
-            A[t] = __fadd_rn(fn[t], al[t]);
+            A[t] = __fadd_rn((float)fn[t], al[t]);
             if constexpr (OPT) A[t] = __fmul_rn(A[t], mk[t]);
             const float4 q = p[t >> 2];
             const float pt = (t & 3) == 0 ? q.x : (t & 3) == 1 ? q.y : (t & 3) == 2 ? q.z : q.w;
@@ -235,7 +239,7 @@ k_sweep_reg(SweepArgs a)
         const int sel = hit ? found : -1;
 #pragma unroll
         for (int t = 0; t < T; ++t)
-            if (sel == t) fn[t] = __fadd_rn(fn[t], WT ? wt : 1.f);
+            if (sel == t) fn[t] += WT ? FT(wt) : FT(1);
         // (predicated: a store under `if` is a branch on the draw's chain)
         asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p st.shared.s32 [%1], %2;\n}"
                      :: "r"((int)hit), "r"((uint32_t)__cvta_generic_to_shared(s_tok + j)), "r"(topic_of(found))
@@ -372,12 +376,12 @@ k_sweep_reg(SweepArgs a)
             for (int t = 0; t < T; ++t) {
                 const int k = topic_of(t);
                 cn[t] = k < K ? grow[k] : 0;
-                fn[t] = (float)cn[t];
+                fn[t] = (FT)cn[t];
             }
             __syncthreads();             // every warp has the row before any of them could write it back
             const uint64_t b = a.doc_off[d];
             const uint32_t L = (uint32_t)(a.doc_off[d + 1] - b);
-            const uint32_t sb = (uint32_t)warp * L / nwarps, se = (uint32_t)(warp + 1) * L / nwarps;
+            const uint32_t sb = (uint32_t)((uint64_t)warp * L / nwarps), se = (uint32_t)((uint64_t)(warp + 1) * L / nwarps);
             const uint32_t m = a.split_step;
             const uint32_t steps = ((L + nwarps - 1) / nwarps + m - 1) / m;   // the longest slice's steps
             uint32_t st = 0;
@@ -389,7 +393,7 @@ k_sweep_reg(SweepArgs a)
                 for (int t = 0; t < T; ++t) {
                     const int k = topic_of(t);
                     if (k < K) cn[t] += d0[k];
-                    fn[t] = (float)cn[t];
+                    fn[t] = (FT)cn[t];
                 }
                 buf = buf == 2 ? 0 : buf + 1;
                 ++st;
@@ -426,7 +430,7 @@ k_sweep_reg(SweepArgs a)
 #pragma unroll
         for (int t = 0; t < T; ++t) {
             const int k = topic_of(t);
-            fn[t] = k < K ? (float)grow[k] : 0.f;
+            fn[t] = k < K ? (FT)grow[k] : FT(0);
         }
         auto none = [] () -> int* { return nullptr; };
         const uint64_t un_end = a.unit_off ? a.unit_off[d + 1] : 1;
