@@ -1024,7 +1024,9 @@ __global__ void k_ll_tab(LlTab t, const float* __restrict__ alpha, uint32_t K, c
 // nonzero, so evaluating them in place cost a warp nearly the whole row; with
 // the tables the counts' bytes bound the kernel.  The terms and their order are
 // the same, so the sums are the same bits.  K = 400, V = 30,000, 10M tokens (125 MB of counts): 200 -> 62 us.
-template <typename CT, typename LT, bool TAB>
+// kUnroll: counts in flight per lane; 1 where a row is no longer than a warp and
+// the others would be tests only (weighted, K = 20, 200,000 documents: ll() 149 us with 8).
+template <typename CT, typename LT, bool TAB, int kUnroll>
 __global__ void k_ll_partials(const CT* __restrict__ ndk, uint64_t D, uint32_t K,
                               const double* __restrict__ lg_alpha, const float* __restrict__ alpha,
                               const LT* __restrict__ doc_len, const double* __restrict__ asum_p,
@@ -1033,7 +1035,6 @@ __global__ void k_ll_partials(const CT* __restrict__ ndk, uint64_t D, uint32_t K
                               const uint32_t* __restrict__ arow, const double* __restrict__ row_asum, LlTab tab)
 {
     __shared__ double s_d[32], s_r[32];
-    constexpr int kUnroll = 8;           // counts in flight per lane
     const double asum = asum_p[0], lg_asum = asum_p[1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -2268,7 +2269,8 @@ void do_ll(tmt_handle* h, double* d_out)
     k_ll_prep<<<1, 256, 0, h->stream>>>(h->d_alpha, K, h->d_lg_alpha, h->d_asum_ll);
     launch_check(h);
     if (h->weighted) {
-        k_ll_partials<float, float, false><<<h->n_partials, 256, 0, h->stream>>>(
+        const auto partials = K <= 32 ? k_ll_partials<float, float, false, 1> : k_ll_partials<float, float, false, 8>;
+        partials<<<h->n_partials, 256, 0, h->stream>>>(
             reinterpret_cast<const float*>(h->d_ndk), h->D, K, h->d_lg_alpha, h->d_alpha, (const float*)h->d_doc_wlen,
             h->d_asum_ll, reinterpret_cast<const float*>(h->d_nkw[0]), h->cfg.V, eta, std::lgamma(eta), h->d_partials,
             h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum, LlTab{});
@@ -2287,19 +2289,22 @@ void do_ll(tmt_handle* h, double* d_out)
         t.doc = h->d_part_nom;
         t.word = t.doc + (uint64_t)t.nd * K;
         t.len = t.word + t.nw;
-        // (not for states whose counts are fewer than the tables' entries)
-        const uint64_t entries = (uint64_t)t.nd * K + t.nw + t.nl;
-        const bool use_tab = entries && rows * K + (uint64_t)K * h->cfg.V >= 4 * entries;
+        // (from 2^20 counts on, where they earn their launch: ll() of 640,000 counts 42 us with
+        // them, 38 without; of 1.04M the same; K = 400, 31M 0.25 -> 0.10 ms)
+        const uint64_t entries = (uint64_t)t.nd * K + t.nw + t.nl, counts = (rows + h->cfg.V) * K;
+        const bool use_tab = entries && counts >= std::max<uint64_t>(1 << 20, 4 * entries);
         const double lg_eta = std::lgamma(eta);
         if (use_tab) {
             k_ll_tab<<<(uint32_t)std::min<uint64_t>((entries + 255) / 256, (uint64_t)h->num_sms * 8), 256, 0, h->stream>>>(
                 t, h->d_alpha, K, h->d_lg_alpha, h->d_asum_ll, eta, lg_eta);
             launch_check(h);
-            k_ll_partials<int32_t, int32_t, true><<<h->n_partials, 256, 0, h->stream>>>(
+            k_ll_partials<int32_t, int32_t, true, 8><<<h->n_partials, 256, 0, h->stream>>>(
                 h->d_ndk, rows, K, h->d_lg_alpha, h->d_alpha, h->d_doc_len, h->d_asum_ll, h->d_nkw[h->cur], h->cfg.V, eta,
                 lg_eta, h->d_partials, h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum, t);
         } else {
-            k_ll_partials<int32_t, int32_t, false><<<h->n_partials, 256, 0, h->stream>>>(
+            const auto partials =
+                K <= 32 ? k_ll_partials<int32_t, int32_t, false, 1> : k_ll_partials<int32_t, int32_t, false, 8>;
+            partials<<<h->n_partials, 256, 0, h->stream>>>(
                 h->d_ndk, rows, K, h->d_lg_alpha, h->d_alpha, h->d_doc_len, h->d_asum_ll, h->d_nkw[h->cur], h->cfg.V, eta,
                 lg_eta, h->d_partials, h->prior_args(), h->d_alpha_rows, h->d_arow, h->d_row_asum, t);
         }
@@ -3511,9 +3516,9 @@ tmt_status tmt_ll_counts_noalloc(const int32_t* n_dk, uint64_t D, uint32_t K, co
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const double etad = (double)eta;
     k_ll_prep<<<1, 256, 0, st>>>(alpha, K, lg_alpha, asum);
-    k_ll_partials<int32_t, int32_t, false><<<blocks, 256, 0, st>>>(n_dk, D, K, lg_alpha, alpha, doc_len, asum, n_kw, V,
-                                                                   etad, std::lgamma(etad), partials, PriorArgs{},
-                                                                   nullptr, nullptr, nullptr, LlTab{});
+    const auto ll_partials = K <= 32 ? k_ll_partials<int32_t, int32_t, false, 1> : k_ll_partials<int32_t, int32_t, false, 8>;
+    ll_partials<<<blocks, 256, 0, st>>>(n_dk, D, K, lg_alpha, alpha, doc_len, asum, n_kw, V, etad, std::lgamma(etad),
+                                        partials, PriorArgs{}, nullptr, nullptr, nullptr, LlTab{});
     k_ll_final<<<1, 256, 0, st>>>(partials, blocks, n_k, K, (double)V * etad, ll_out, nullptr);
     // no error was pending before the launches: one now is theirs
     e = cudaGetLastError();
