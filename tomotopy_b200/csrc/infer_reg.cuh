@@ -1,6 +1,6 @@
-// infer_reg.cuh -- inference of unseen documents for K <= kInferRegMaxK.
-// Included by infer.cuh inside tmtk, after InferArgs; k_infer_slots there is
-// the kernel of larger K and states the computation.  Both give the same
+// infer_reg.cuh -- inference of unseen documents for K <= kInferRegMaxK, included by
+// infer_k256.cu, infer_k512.cu and infer_k1024.cu.  k_infer_slots (infer.cu) is the
+// kernel of larger K; infer.cuh states the computation.  Both give the same
 // results, bit for bit.
 //
 // What bounds it: a document is one warp's chain of draws (its tokens times its
@@ -21,8 +21,11 @@
 // One document of 250 tokens, K = 100, 50 sweeps: 14.4 -> 4.8 ms; 4,096 documents
 // 312 -> 137 ms; 1,024 documents at K = 1000 146 -> 69 ms.
 
-constexpr uint32_t kInferRegMaxK = 1024;
-constexpr int kInferRegWarps = 4;    // warps (documents) per block: one per SM sub-partition
+#pragma once
+#include <algorithm>
+#include "infer_doc.cuh"
+
+namespace tmtk {
 
 // resident blocks per SM (registers a thread may use), as many as leave the draws
 // (nearly) without spills and as the arrays' shared memory admits
@@ -577,3 +580,37 @@ k_infer_reg(InferArgs a)
         finish_doc<WT>(a, sl, b, L, WT ? wsum : (float)nvalid, lane, s_own, [&](int k) -> CT { return s_n[at(k)]; });
     }
 }
+
+template <int CH, int STEPS, bool WT, int MODE>
+inline void launch_infer_reg_t(const InferArgs& a, int num_sms, cudaStream_t st)
+{
+    auto kern = k_infer_reg<CH, STEPS, WT, MODE>;
+    const uint32_t smem = (4 + kInferRegWarps * (!WT && CH <= 4 ? 6 : 4)) * 4 * 128 * CH;     // (k_infer_reg's s_dyn)
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kInferRegWarps * 32, smem));
+    if (per_sm < 1) throw CudaError("infer kernel does not fit on an SM");
+    const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)per_sm * num_sms,
+                                                                          (a.n_work + kInferRegWarps - 1) / kInferRegWarps));
+    kern<<<grid, kInferRegWarps * 32, smem, st>>>(a);
+    CK(cudaGetLastError());
+}
+
+template <int CH, int STEPS, bool WT>
+inline void launch_infer_reg_g(const InferArgs& a, int num_sms, cudaStream_t st)
+{
+    // The fast modes' conditions: scalar eta, counts exact in to_f, denominators in
+    // recip's range.  (Their general forms cost a draw at k = 100 about 50 of 450
+    // cycles.)  Element loads where columns are not 16-byte aligned.
+    // (No weight or sum of weights can overflow: A B R below 1e36 / K.  With V eta at
+    // most 1e30 this also keeps weighted counts below 1e31, inside recip's range.)
+    const double most = WT ? a.count_max : 8388608.0;
+    const bool finite = (most + (double)a.asum_f) * (most + (double)a.eta) < 1e32 * (double)a.veta;
+    const bool exact = WT || a.count_max < 8388608.0;
+    if (a.pidx || !exact || !finite || !(a.veta >= 1e-30f && a.veta <= 1e30f))
+        launch_infer_reg_t<CH, 5, WT, 2>(a, num_sms, st);
+    else if (a.K & 3) launch_infer_reg_t<CH, STEPS, WT, 1>(a, num_sms, st);
+    else launch_infer_reg_t<CH, STEPS, WT, 0>(a, num_sms, st);
+}
+
+} // namespace tmtk
