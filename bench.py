@@ -49,12 +49,11 @@ def bytes_per_sweep(N, K, V):
     return N * (4 * K + 16) + 8 * K * V + 4 * (V + 1) + 8 * K
 
 
-# DRAM bytes of one sweep of k_sweep_doc (which ran K = 1000 before k_sweep_wide) measured by ncu outside the bench (dram__bytes_read.sum +
-# dram__bytes_write.sum), keyed by config: shown beside the roofline as the
-# capture it came from; the bench itself measures no DRAM traffic, so its
-# roofline.traffic stays null.
-NCU_TRAFFIC = {"c3": {"bytes_per_sweep": 108.3e9 + 9.6e9,
-                      "source": "profiles/k_sweep_doc_c3_traffic.md (100k-document capture scaled by tokens, "
+# DRAM bytes of one sweep, measured by ncu outside the bench, keyed by config: shown
+# beside the roofline as the capture it came from; the bench itself measures no
+# DRAM traffic, so its roofline.traffic stays null.
+NCU_TRAFFIC = {"c3": {"bytes_per_sweep": 116.5e9 + 9.6e9,
+                      "source": "profiles/k_sweep_wide_c3.md (capture of a launch of 3M tokens scaled by tokens, "
                                 "plus k_phi_copy)"}}
 
 

@@ -515,7 +515,7 @@ struct SweepArgs {
     uint32_t rowi_smem;      // 1: the int n_dk row lives in shared memory
     uint32_t dnk_smem;       // 1: n_k deltas aggregate in shared memory
     // split documents: positions [pos_begin, pos_begin + n_long) are sampled
-    // one per block in slices (phase 1 of k_sweep_doc); 0: none
+    // one per block in slices (phase 1 of k_sweep_reg); 0: none
     uint32_t n_long;
     uint32_t split_step;     // positions per slice between merges
     uint32_t* long_counter;  // phase 1's document counter
@@ -1278,7 +1278,7 @@ k_alpha_sums(const CT* __restrict__ ndk, uint64_t D, uint32_t K, const float* __
 // 64 threads adding its topic's partial sums in order (16 loads in flight), a third
 // warp meanwhile the length sums; the last block to finish forms the new
 // sum(alpha), in order.  Bound by the chain of dependent FP64 adds.  (One block for all
-// topics, its serial sums read from global memory: 118 us at 592 partial sums; now 32.)
+// topics, its serial sums read from global memory: K = 200, 592 partial sums 116 us, now 56.)
 constexpr uint32_t kAlphaUpd = 64;
 
 __global__ void __launch_bounds__(kAlphaUpd + 32)
@@ -1405,7 +1405,7 @@ struct tmt_handle {
     float* d_rm1 = nullptr;          // K: the own topic's reciprocal of the snapshot
     uint32_t groups = 1;             // document groups per sweep
     std::vector<uint64_t> group_bounds;   // doc_order positions: group g = [b[g], b[g+1])
-    // long documents (k_sweep_doc phase 1): per group, the tokens of the
+    // long documents (k_sweep_reg, phase 1): per group, the tokens of the
     // global group, and the number of its first (longest) local documents
     // that are split; the lengths of the local documents in doc_order
     std::vector<uint64_t> group_tokens;
@@ -1936,8 +1936,11 @@ void launch_wide_ch(tmt_handle* h, const SweepArgs& a)
 void launch_sweep(tmt_handle* h, const SweepArgs& a, int variant)
 {
     // k_sweep_wide above kRegMaxK, and from 257 topics on where the launch has documents
-    // enough (16 an SM) that instructions bound it, not the chain of the longest: K = 333,
-    // 4.9M tokens, 10 sweeps 28.1 -> 26.9 ms (at K = 130, 17.9 -> 19.7: not below 257)
+    // enough (16 an SM) that instructions bound it, not the chain of the longest: measured at
+    // K = 333 with short documents (4.9M tokens, 10 sweeps 28.1 -> 26.9 ms) and at K = 130
+    // (17.9 -> 19.7: not below 257).  The count of documents stands for their lengths,
+    // which it does not see: weighted documents are never split, so a launch of many of them goes
+    // here however long its longest.
     if (a.K <= kWideMaxK &&
         (a.K > kRegMaxK || (a.K > 256 && !a.n_long && a.pos_end - a.pos_begin >= (uint64_t)h->num_sms * 16))) {
         if (a.K <= 384) launch_wide_ch<3>(h, a);

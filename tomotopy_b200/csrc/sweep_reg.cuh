@@ -1,7 +1,7 @@
 // sweep_reg.cuh -- the training sweep for K <= 512 (K <= kRegMaxK): the
 // document's row in registers.  Included by engine.cu inside its namespace,
-// after SweepArgs; k_sweep_doc there is the kernel of larger K and states the
-// sampler.  Both compute the same draws, bit for bit.
+// after SweepArgs; k_sweep_doc there, the kernel of K > 1024, states the sampler
+// (k_sweep_wide is the one between).  All compute the same draws, bit for bit.
 //
 // What bounds it: a document is a chain of draws, each token waiting for the
 // one before, so a launch of few or long documents lasts (longest document) x
@@ -18,8 +18,9 @@
 // two ahead of the draws; the words' table columns are loaded kRing - 1 tokens
 // ahead.  (Products with a 0/1 vector in place of the own topic's selects, and split
 // merges through per-warp buffers in place of shared-memory atomics, measured slower.)
-// 10 sweeps, k_sweep_doc before and this kernel: K = 20, 1.5M tokens 13.5 -> 5.2 ms;
-// K = 100, 27.5M tokens 93 -> 52.5 ms; IDF weights, K = 200, 8M tokens 137 -> 57 ms.
+// The sampling kernels of one sweep, k_sweep_doc and this kernel: K = 20, 1.5M tokens 1.33 ->
+// 0.45 ms; K = 100, 27.5M tokens 8.5 -> 4.7 ms; IDF weights, K = 200, 8M tokens 12.6 -> 4.6 ms
+// (2.5 of them the launch of the 10,000-token documents).
 
 constexpr uint32_t kRegMaxK = 512;
 constexpr uint64_t kRegFloatLen = 1ull << 24;    // counts below are exact as floats
@@ -140,6 +141,7 @@ k_sweep_reg(SweepArgs a)
         ri1 = 0.f;
         vm1 = __ballot_sync(FULL, w1 < a.V);
         if (w1 < a.V) {
+            // (32 bits: V K below 2^34; the counts' 12 bytes an entry end a device's memory before)
             s_col[(col_end + __popc(vm1 & lt)) & 63] = w1 * (uint32_t)(KP >> 2);
             nkw1 = __ldg(reinterpret_cast<const CT*>(a.nkw) + (uint64_t)w1 * K + z1);
             ri1 = __ldg((WT ? reinterpret_cast<const float*>(a.nk) : a.rm1) + z1);

@@ -9,12 +9,14 @@
 // 281 warp instructions a token and waited for each new column.  Here the next
 // token's column is loaded as soon as the hit lane has handed its part of the
 // current one to the second scan, so the second scan and the update hide the load
-// (a second buffer in registers hid it too, but at 16 warps an SM: 198 against 186 ms
-// below); token scalars, own-topic weights and count deltas are formed for 32 tokens
+// (a second buffer in registers hid it too, but at 16 warps an SM: K = 1000, 24M tokens,
+// 10 sweeps with the state read back 198 against 186 ms); token scalars, own-topic weights and count deltas are formed for 32 tokens
 // at a time (as in k_sweep_reg); the row's updates are predicated stores; the
 // row is padded with zeros to 128 CH topics and CH is exact, so the fma chain has no
-// guards.  K = 1000, 24M tokens, 10 sweeps with the state read back (25 ms):
-// 205.6 -> 186.4 ms.
+// guards.  The sampling kernels of one sweep, k_sweep_doc's faster variant and this kernel: K = 1000,
+// 24M tokens 15.7 -> 14.2 ms, 4.6 -> 3.4 of it the launch of the longest documents; 204M
+// tokens, where that launch weighs little, 90.6 -> 90.4 ms, but without the tuner's sweeps
+// of a slower variant.
 
 constexpr uint32_t kWideMaxK = 1024;
 constexpr int kWideWarps = 4;
@@ -109,6 +111,7 @@ k_sweep_wide(SweepArgs a)
         ri1 = 0.f;
         vm1 = __ballot_sync(FULL, w1 < a.V);
         if (w1 < a.V) {
+            // (32 bits: V K below 2^34; the counts' 12 bytes an entry end a device's memory before)
             s_col[(col_end + __popc(vm1 & lt)) & 63] = w1 * (uint32_t)(KP >> 2);
             nkw1 = __ldg(reinterpret_cast<const CT*>(a.nkw) + (uint64_t)w1 * K + z1);
             ri1 = __ldg((WT ? reinterpret_cast<const float*>(a.nk) : a.rm1) + z1);
